@@ -135,22 +135,24 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bf
 }
 
 // gate_up [T, 2I] -> act(gate) * up, bf16 or fp8+scale.  ACT 0: SiLU, 1: tanh-approximated GELU (Gemma).
+// `rows` (expert-sorted buffers): block i works on row rows[i], or on nothing where that is negative, so that the padding of
+// the experts' tiles costs nothing (48 tokens on 512 experts: 70 us over all padded rows, 3.3 us over the 480 live ones).
 template <int ACT>
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const __nv_bfloat16* __restrict__ gu, long long ld, int I, __nv_bfloat16* y, long long ldy, uint8_t* q,
-                long long ldq, float* scale, long long scale_ld, const int* live_tiles) {
+                long long ldq, float* scale, long long scale_ld, const int* rows) {
   chain_trigger();
   chain_wait();
-  const int t = blockIdx.x;           // rows on grid.x: row counts can exceed the 65535 limit of grid.y
-  if (live_tiles && t >= (*live_tiles) * 128) return;      // expert-sorted buffers: rows past the live tiles are unused
+  const int t = rows ? rows[blockIdx.x] : (int)blockIdx.x;      // rows on grid.x: row counts can exceed the 65535 limit of grid.y
+  if (t < 0) return;
   const int e = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
   const bool live = e < I;
   float o[8];
   float amax = 0.f;
   if (live) {
     float g[8], u[8];
-    load8(gu + t * ld + e, g);
-    load8(gu + t * ld + I + e, u);
+    load8(gu + (long long)t * ld + e, g);
+    load8(gu + (long long)t * ld + I + e, u);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       float s;
@@ -688,14 +690,16 @@ extern "C" int atlas_rmsnorm(const void* x, long long ldx, const void* residual,
   return cudaGetLastError() == cudaSuccess ? 0 : -20;
 }
 
+// `rows` (device, T entries; may be null): the row of gu, y and q that each block takes, negative for none
 extern "C" int atlas_silu_mul(const void* gu, long long ld, int T, int I, void* y, long long ldy, void* q,
-                              long long ldq, float* scale, long long scale_ld, const int* live_tiles, void* stream) {
+                              long long ldq, float* scale, long long scale_ld, const int* rows, void* stream) {
   if (T <= 0) return 0;
   if (I % 8 || (q && I % 128)) return -1;
-  dim3 grid(T, (I / 8 + 255) / 256);
-  launch_chain_if(T <= 256, silu_mul_kernel<0>, grid, dim3(256), 0, reinterpret_cast<cudaStream_t>(stream),
+  const int threads = min(256, (I / 8 + 31) / 32 * 32);      // whole warps: groups of 16 lanes share a scale
+  dim3 grid(T, (I / 8 + threads - 1) / threads);
+  launch_chain_if(T <= 256, silu_mul_kernel<0>, grid, dim3(threads), 0, reinterpret_cast<cudaStream_t>(stream),
       reinterpret_cast<const __nv_bfloat16*>(gu), ld, I, reinterpret_cast<__nv_bfloat16*>(y), ldy,
-      reinterpret_cast<uint8_t*>(q), ldq, scale, scale_ld, live_tiles);
+      reinterpret_cast<uint8_t*>(q), ldq, scale, scale_ld, rows);
   return cudaGetLastError() == cudaSuccess ? 0 : -20;
 }
 

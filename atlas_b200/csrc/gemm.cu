@@ -127,6 +127,7 @@ struct GemmParams {
   // what the fold needs.
   unsigned long long* timeline;
   const int* tile_expert;       // nullptr = plain GEMM
+  const int* tile_rows;         // live rows of every tile, its leading ones: the others are neither copied nor stored
   const int* num_m_tiles_ptr;   // device-side tile count (the host cannot know it)
   int expert_n;                 // output features per expert
   long long b_scale_expert_stride;
@@ -446,17 +447,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const int split = ip.split;
         const int kb0 = split * p.kb_per_split;
         const int kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
+        // expert tiles: as many copies of a_box_rows rows as the tile's live rows take
+        const int a_rows = p.tile_rows ? (p.tile_rows[m_tile] + p.a_box_rows - 1) / p.a_box_rows * p.a_box_rows : p.a_box_rows;
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, 0x100)) { ok = false; break; }
           uint8_t* sa = smem + stage * Cfg::kStageBytes;
-          mbar_expect_tx(&full[stage], p.a_box_rows * kRowBytes + Cfg::kBBytes);
+          mbar_expect_tx(&full[stage], a_rows * kRowBytes + Cfg::kBBytes);
           if (FP8) {
             mbar_expect_tx(&sc_full[sc_slot], kBlockM * 4);
             bulk_g2s(sc_ring + sc_slot * kBlockM, p.a_scale + (long long)kb * p.sa_k + m_tile * kBlockM, kBlockM * 4,
                      &sc_full[sc_slot]);
             if (++sc_slot == kScaleSlots) sc_slot = 0;
           }
-          tma_load_2d(sa, &tmap_a, &full[stage], kb * kElemsPerRow, m_tile * kBlockM);
+          for (int r = 0; r < a_rows; r += p.a_box_rows)
+            tma_load_2d(sa + r * kRowBytes, &tmap_a, &full[stage], kb * kElemsPerRow, m_tile * kBlockM + r);
           if (p.epi_mode == 1) {
             // 32-row chunks, gate and up alternating, so that an epilogue thread's 64 columns are 32 gate values and
             // the 32 up values of the same activation columns (the tensor map of B has a 32-row box in this mode)
@@ -1012,7 +1016,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
         asm volatile("bar.sync 1, %0;\n" ::"n"(32 * kEpiWarps));
       } else
-      if (store_now && m < M_rows) {
+      if (store_now && m < (p.tile_rows ? m_tile * kBlockM + p.tile_rows[m_tile] : M_rows)) {
         __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)m * p.ldc;
         if (!FP8 && p.bias != nullptr) {
 #pragma unroll
@@ -1459,12 +1463,12 @@ extern "C" int atlas_gemm_fused(int kind, const void* A, const void* B, void* C,
 
 // Grouped (MoE) GEMM: C[r, :] = A[r, :] * B[e(r)]^T for expert-sorted rows.  `A` has `max_rows` rows (a multiple of
 // 128); m-tile i covers rows [128 i, 128 i + 128) and uses expert tile_expert[i]; *num_m_tiles (device memory) says how
-// many tiles are live.  `B` is the expert stack [E * N, K]; b_scale is [E, ceil(N/128), K/128].  act (bf16): see
-// atlas_gemm_bias_act.
+// many tiles are live and tile_rows[i] how many of a tile's rows.  `B` is the expert stack [E * N, K]; b_scale is
+// [E, ceil(N/128), K/128].  act (bf16): see atlas_gemm_bias_act.  `rows_hint`: rows an expert gets on average.
 extern "C" int atlas_gemm_grouped(int kind, const void* A, const void* B, void* C, const float* a_scale, long long sa_k,
                                   const float* b_scale, int max_rows, int N, int K, int E, long long lda, long long ldb,
-                                  long long ldc, int block_n, const int* tile_expert, const int* num_m_tiles,
-                                  int num_sms, unsigned long long* status, void* stream, int act, float glu_limit,
+                                  long long ldc, int block_n, const int* tile_expert, const int* tile_rows, const int* num_m_tiles,
+                                  int rows_hint, int num_sms, unsigned long long* status, void* stream, int act, float glu_limit,
                                   float glu_alpha, float glu_shift) {
   if (act < 0 || act > 2 || (act && kind != 0)) return -11;
   if (max_rows <= 0 || N <= 0 || K <= 0 || E <= 0) return 0;
@@ -1476,14 +1480,19 @@ extern "C" int atlas_gemm_grouped(int kind, const void* A, const void* B, void* 
   if (kind == 1 && (K % 128)) return -3;
   if (block_n != 64 && block_n != 128 && block_n != 256) return -4;
   if (N % block_n) return -10;            // a tile must not straddle two experts' rows of B
+  if (!tile_rows) return -12;
   CUtensorMap ta, tb;
-  int rc = make_tmap_kmajor(&ta, A, max_rows, K, lda, kBlockM, esize);
+  // Rows per copy of A: padding rows that a copy carries cost ingest (~50 bytes per clock and SM, shared with the weights),
+  // copies cost issue slots of the producer thread.  48 tokens on 512 experts (0.9 rows on average, 1.5 in those that get any): 176 us per
+  // product with whole 128-row copies and stores, 110 us with 8-row copies and the live rows stored.
+  const int a_box = rows_hint < 4 ? 8 : (rows_hint < 12 ? 16 : 32);
+  int rc = make_tmap_kmajor(&ta, A, max_rows, K, lda, a_box, esize);
   if (rc) return rc;
   rc = make_tmap_kmajor(&tb, B, (uint64_t)E * N, K, ldb, block_n, esize);
   if (rc) return rc;
   GemmParams p = {};
   p.timeline = g_gemm_timeline;
-  p.a_box_rows = kBlockM;
+  p.a_box_rows = a_box; p.tile_rows = tile_rows;
   p.C = C; p.a_scale = a_scale; p.b_scale = b_scale; p.workspace = nullptr; p.counters = nullptr;
   p.status = status; p.ldc = ldc; p.sa_k = sa_k; p.M = max_rows; p.N = N; p.K = K;
   p.k_blocks = (K + elems_per_row - 1) / elems_per_row;

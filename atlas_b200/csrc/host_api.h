@@ -45,7 +45,7 @@ int atlas_rmsnorm(const void* x, long long ldx, const void* residual, long long 
                   long long ldro, void* y, long long ldy, void* q, long long ldq, float* scale, long long scale_ld,
                   int T, int H, float eps, int plus_one, void* stream);
 int atlas_silu_mul(const void* gu, long long ld, int T, int I, void* y, long long ldy, void* q, long long ldq,
-                   float* scale, long long scale_ld, const int* live_tiles, void* stream);
+                   float* scale, long long scale_ld, const int* rows, void* stream);
 int atlas_quant_fp8(const void* x, long long ld, int T, int K, void* q, long long ldq, float* scale,
                     long long scale_ld, void* stream);
 int atlas_rope_kv_write(void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv,
@@ -66,9 +66,9 @@ int atlas_moe_route_ex(const void* logits, long long ld, int is_bf16, int T, int
                        const float* sel_bias, int n_group, int topk_group, const int* hash_table, const int* token_ids,
                        float out_scale, float* w_out, int* id_out, void* stream);
 int atlas_moe_align(const int* topk_ids, int T, int k, int e_lo, int E_local, int* slot_of, int* row_token,
-                    int* tile_expert, int* num_tiles, int max_rows, unsigned long long* status, void* stream);
-int atlas_moe_gather(const void* x, long long ldx, const int* row_token, const int* num_tiles, int max_rows, int H,
-                     void* y, void* q, float* scale, long long scale_ld, void* stream);
+                    int* tile_expert, int* tile_rows, int* num_tiles, int max_rows, unsigned long long* status, void* stream);
+int atlas_moe_gather(const void* x, long long ldx, const int* slot_of, int T, int k, int H, void* y, void* q, float* scale,
+                     long long scale_ld, void* stream);
 int atlas_moe_combine(const void* y, long long ldy, const int* slot_of, const float* topk_w, int T, int k, int H,
                       const void* addend, long long ld_add, void* out, long long ldo, void* stream);
 int atlas_moe_dispatch_prep(const int* topk_ids, int pairs, int experts_per_rank, int world, int* send_off, int* pos,
@@ -86,8 +86,8 @@ int atlas_gemm_w4a16_grouped(const void* A, const void* packed, const void* bsca
                              void* stream);
 int atlas_gemm_grouped(int kind, const void* A, const void* B, void* C, const float* a_scale, long long sa_k,
                        const float* b_scale, int max_rows, int N, int K, int E, long long lda, long long ldb,
-                       long long ldc, int block_n, const int* tile_expert, const int* num_m_tiles, int num_sms,
-                       unsigned long long* status, void* stream, int act, float glu_limit, float glu_alpha, float glu_shift);
+                       long long ldc, int block_n, const int* tile_expert, const int* tile_rows, const int* num_m_tiles,
+                       int rows_hint, int num_sms, unsigned long long* status, void* stream, int act, float glu_limit, float glu_alpha, float glu_shift);
 int atlas_gemm_bias_act(const void* A, const void* B, void* C, float* tail, long long tail_ld, int n_main, const float* bias, int act,
                         float glu_limit, float glu_alpha, float glu_shift, int M, int N, int K, long long lda, long long ldb, long long ldc, int block_n, int splits, float* workspace, int* counters, int num_sms,
                         unsigned long long* status, void* stream);

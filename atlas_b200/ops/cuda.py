@@ -229,7 +229,7 @@ def rmsnorm(x, w, eps, residual=None, plus_one=False, quant=False):
     return y, res_out
 
 
-def silu_mul(gate_up: torch.Tensor, quant=False, live_tiles: Optional[torch.Tensor] = None):
+def silu_mul(gate_up: torch.Tensor, quant=False):
     assert gate_up.dtype == torch.bfloat16 and gate_up.stride(1) == 1
     T, I2 = gate_up.shape
     I = I2 // 2
@@ -238,10 +238,10 @@ def silu_mul(gate_up: torch.Tensor, quant=False, live_tiles: Optional[torch.Tens
         q = torch.empty(T, I, dtype=FP8, device=gate_up.device)
         s = _scale_buf(T, I // 128, gate_up.device)
         _check(lib().atlas_silu_mul(gate_up.data_ptr(), gate_up.stride(0), T, I, None, 0, q.data_ptr(), I, s.data_ptr(),
-                                    s.stride(1), _ptr(live_tiles), _stream()), "silu_mul")
+                                    s.stride(1), None, _stream()), "silu_mul")
         return q, s
     y = torch.empty(T, I, dtype=gate_up.dtype, device=gate_up.device)
-    _check(lib().atlas_silu_mul(gate_up.data_ptr(), gate_up.stride(0), T, I, y.data_ptr(), I, None, 0, None, 0, _ptr(live_tiles), _stream()),
+    _check(lib().atlas_silu_mul(gate_up.data_ptr(), gate_up.stride(0), T, I, y.data_ptr(), I, None, 0, None, 0, None, _stream()),
            "silu_mul")
     return y
 

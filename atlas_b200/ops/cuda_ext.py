@@ -15,10 +15,10 @@ FP8 = torch.float8_e4m3fn
 
 def bind(lib) -> None:
     lib.atlas_moe_route.argtypes = [_vp, _ll, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp]
-    lib.atlas_moe_align.argtypes = [_vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _vp, _vp]
-    lib.atlas_moe_gather.argtypes = [_vp, _ll, _vp, _vp, _i, _i, _vp, _vp, _vp, _ll, _vp]
+    lib.atlas_moe_align.argtypes = [_vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp, _vp]
+    lib.atlas_moe_gather.argtypes = [_vp, _ll, _vp, _i, _i, _i, _vp, _vp, _vp, _ll, _vp]
     lib.atlas_moe_combine.argtypes = [_vp, _ll, _vp, _vp, _i, _i, _i, _vp, _ll, _vp, _ll, _vp]
-    lib.atlas_gemm_grouped.argtypes = [_i, _vp, _vp, _vp, _vp, _ll, _vp, _i, _i, _i, _i, _ll, _ll, _ll, _i, _vp, _vp, _i, _vp, _vp, _i, _f, _f, _f]
+    lib.atlas_gemm_grouped.argtypes = [_i, _vp, _vp, _vp, _vp, _ll, _vp, _i, _i, _i, _i, _ll, _ll, _ll, _i, _vp, _vp, _vp, _i, _i, _vp, _vp, _i, _f, _f, _f]
     lib.atlas_moe_plain_gemm.argtypes = [_vp, _ll, _vp, _vp, _vp, _vp, _i, _i, _i, _f, _f, _f, _i, _i, _vp, _ll, _i, _vp]
     lib.atlas_moe_plain_combine.argtypes = [_vp, _ll, _vp, _vp, _i, _i, _i, _vp, _ll, _i, _vp]
     lib.atlas_moe_dispatch_prep.argtypes = [_vp, _i, _i, _i, _vp, _vp, _vp]
@@ -305,15 +305,16 @@ def _moe_local(x, topk_w, topk_ids, experts, e_lo, addend: Optional[torch.Tensor
         kind, w13, s13, w2, s2 = _expert_stacks(experts)
         I = w2.shape[2] * 2 if kind == 2 else w2.shape[2]
         N1 = w13.shape[1]
-    max_rows = ((T * k + E * 127 + 127) // 128) * 128
-    max_rows = min(max_rows, ((T * k + 127) // 128 + E) * 128)
+    # every expert that gets rows has at most one tile that is not full
+    max_tiles = T * k // 128 + min(T * k, E)
+    max_rows = max_tiles * 128
     lib, st, sms, status = K.lib(), K._stream(), K._num_sms[d], K._status_ptr[d]
     slot_of = torch.empty(T * k, dtype=torch.int32, device=dev)
     row_token = torch.empty(max_rows, dtype=torch.int32, device=dev)
-    tile_expert = torch.empty(max_rows // 128, dtype=torch.int32, device=dev)
+    tile_expert, tile_rows = torch.empty(2, max_tiles, dtype=torch.int32, device=dev)
     num_tiles = torch.empty(1, dtype=torch.int32, device=dev)
     K._check(lib.atlas_moe_align(topk_ids.data_ptr(), T, k, e_lo, E, slot_of.data_ptr(), row_token.data_ptr(),
-                                 tile_expert.data_ptr(), num_tiles.data_ptr(), max_rows, status, st), "moe_align")
+                                 tile_expert.data_ptr(), tile_rows.data_ptr(), num_tiles.data_ptr(), max_rows, status, st), "moe_align")
 
     def bn_for(n):
         return 128 if n % 128 == 0 else 64
@@ -346,12 +347,12 @@ def _moe_local(x, topk_w, topk_ids, experts, e_lo, addend: Optional[torch.Tensor
     if kind == 1:
         xq = torch.empty(max_rows, H, dtype=FP8, device=dev)
         xs = torch.empty(H // 128, max_rows, dtype=torch.float32, device=dev)
-        K._check(lib.atlas_moe_gather(x.data_ptr(), x.stride(0), row_token.data_ptr(), num_tiles.data_ptr(), max_rows, H,
+        K._check(lib.atlas_moe_gather(x.data_ptr(), x.stride(0), slot_of.data_ptr(), T, k, H,
                                       None, xq.data_ptr(), xs.data_ptr(), max_rows, st), "moe_gather")
         a1, a1s = xq, xs
     else:
         xp = torch.empty(max_rows, H, dtype=torch.bfloat16, device=dev)
-        K._check(lib.atlas_moe_gather(x.data_ptr(), x.stride(0), row_token.data_ptr(), num_tiles.data_ptr(), max_rows, H,
+        K._check(lib.atlas_moe_gather(x.data_ptr(), x.stride(0), slot_of.data_ptr(), T, k, H,
                                       xp.data_ptr(), None, None, 0, st), "moe_gather")
         a1, a1s = xp, None
     fused_act = _EXPERT_ACTS.get(activation, 0) if kind == 0 else 0       # bf16 experts: part of the product's epilogue
@@ -364,20 +365,20 @@ def _moe_local(x, topk_w, topk_ids, experts, e_lo, addend: Optional[torch.Tensor
     else:
         K._check(lib.atlas_gemm_grouped(kind, a1.data_ptr(), w13.data_ptr(), h1.data_ptr(), K._ptr(a1s), max_rows, K._ptr(s13),
                                         max_rows, N1, H, E, H, H, N1o, bn_for(N1), tile_expert.data_ptr(),
-                                        num_tiles.data_ptr(), sms, status, st, fused_act, *_unit(unit)), "moe_gemm1")
+                                        tile_rows.data_ptr(), num_tiles.data_ptr(), T * k // E, sms, status, st, fused_act, *_unit(unit)), "moe_gemm1")
     if own_act:
         act = h1 if fused_act else (K.relu_squared(h1) if activation == "relu2" else K.gated_unit(h1, unit, paired=True))
         a2, a2s = K.quant_fp8(act) if kind == 1 else (act, None)
     elif kind == 1:
         aq = torch.empty(max_rows, I, dtype=FP8, device=dev)
         asc = torch.empty(I // 128, max_rows, dtype=torch.float32, device=dev)
-        K._check(lib.atlas_silu_mul(h1.data_ptr(), 2 * I, max_rows, I, None, 0, aq.data_ptr(), I, asc.data_ptr(), max_rows,
-                                    num_tiles.data_ptr(), st), "moe_silu")
+        K._check(lib.atlas_silu_mul(h1.data_ptr(), 2 * I, T * k, I, None, 0, aq.data_ptr(), I, asc.data_ptr(), max_rows,
+                                    slot_of.data_ptr(), st), "moe_silu")
         a2, a2s = aq, asc
     else:
         act = torch.empty(max_rows, I, dtype=torch.bfloat16, device=dev)
-        K._check(lib.atlas_silu_mul(h1.data_ptr(), 2 * I, max_rows, I, act.data_ptr(), I, None, 0, None, 0,
-                                    num_tiles.data_ptr(), st), "moe_silu")
+        K._check(lib.atlas_silu_mul(h1.data_ptr(), 2 * I, T * k, I, act.data_ptr(), I, None, 0, None, 0,
+                                    slot_of.data_ptr(), st), "moe_silu")
         a2, a2s = act, None
     y = torch.empty(max_rows, H, dtype=torch.bfloat16, device=dev)
     if kind == 2:
@@ -386,8 +387,8 @@ def _moe_local(x, topk_w, topk_ids, experts, e_lo, addend: Optional[torch.Tensor
                                               sms, status, st), "moe_gemm2_w4")
     else:
         K._check(lib.atlas_gemm_grouped(kind, a2.data_ptr(), w2.data_ptr(), y.data_ptr(), K._ptr(a2s), max_rows, K._ptr(s2),
-                                        max_rows, H, I, E, I, I, H, bn_for(H), tile_expert.data_ptr(), num_tiles.data_ptr(),
-                                        sms, status, st, 0, 0.0, 0.0, 0.0), "moe_gemm2")
+                                        max_rows, H, I, E, I, I, H, bn_for(H), tile_expert.data_ptr(),
+                                        tile_rows.data_ptr(), num_tiles.data_ptr(), T * k // E, sms, status, st, 0, 0.0, 0.0, 0.0), "moe_gemm2")
     if rows_ok and addend is None:
         return ExpertRows(y, slot_of, topk_w)
     return _finish(lib, y, slot_of, topk_w, T, k, H, addend, fused_comm, grouped, dev, st)
