@@ -17,7 +17,7 @@ import torch
 from .config import EngineConfig
 from .layers import LatentAttention
 from .models import CacheStore, DecoderLM, ForwardBatch
-from .models.decoder import attention_of, recurrent_of
+from .models.decoder import attention_of
 from .sched import SchedulerOutput
 
 _PIN_RING = 3              # staging buffers per tensor: how many steps the host may run ahead
@@ -44,9 +44,6 @@ class ModelRunner:
         self.graph_replays = 0
         self._pin: Dict[str, list] = {}              # per name: a ring of (pinned buffer, event after its last copy)
         self._pin_turn: Dict[str, int] = {}
-        # decode graphs of recurrent models read state slots from a device buffer; the kernels that take everything they
-        # need from there are those of recurrent.cu
-        self._states_graph_safe = all(l.kind != "gdn" for l in model.layers if recurrent_of(l) is not None)
         # slot of padding rows: the last one, which the engine allocates beyond those it hands out
         self.pad_state_slot = next((t.shape[0] - 1 for st in cache.states.values() for t in st.values()), None)
         if self.on_gpu:
@@ -243,7 +240,7 @@ class ModelRunner:
         return (self.on_gpu and self.cfg.use_cuda_graphs and batch.num_seqs > 0
                 and batch.num_decodes == batch.num_seqs and not batch.spec_verify and batch.adapter_rows is None
                 and batch.positions3 is None
-                and getattr(self.model, "graph_safe", True) and self._states_graph_safe and not batch.snapshot_plan
+                and getattr(self.model, "graph_safe", True) and not batch.snapshot_plan
                 and all(batch.has_state_host))
 
     def forward(self, batch: ForwardBatch) -> torch.Tensor:

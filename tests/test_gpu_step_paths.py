@@ -1,0 +1,122 @@
+"""Kernels and dispatch rules of prefill and decode steps at the sizes where they can go wrong, on the GPU."""
+import pytest
+import torch
+
+from atlas_b200 import quant as Q
+from atlas_b200.config import PRESETS, EngineConfig
+from atlas_b200.engine import LLMEngine
+from atlas_b200.layers.moe import ExpertWeights
+from atlas_b200.models import ForwardBatch, build_model
+from atlas_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _rel(a, b):
+    a, b = a.double(), b.double()
+    return float((a - b).norm() / b.norm().clamp_min(1e-30))
+
+
+@pytest.fixture(scope="module")
+def K():
+    from atlas_b200.ops import cuda as k
+    k.load()
+    return k
+
+
+# ----------------------------------------------------------------------------- experts on live rows
+def _fp8(x):
+    q, s = Q.per_token_group_quant_fp8(x)
+    return (q.float().view(x.shape[0], -1, 128) * s[..., None]).view(x.shape)
+
+
+def _fp8_experts(x, ex, w, ids, lo):
+    """The weighted sum over a token's experts, with activations rounded to FP8 and intermediate rows to bf16."""
+    w13, w2 = ex.dequantized()
+    y, xq = torch.zeros(x.shape, device=DEV), _fp8(x)
+    for e in range(w13.shape[0]):
+        t, j = (ids == e + lo).nonzero(as_tuple=True)
+        if t.numel():
+            g, u = (xq[t] @ w13[e].float().t()).bfloat16().float().chunk(2, -1)
+            o = _fp8((torch.nn.functional.silu(g) * u).bfloat16()) @ w2[e].float().t()
+            y.index_add_(0, t, o.bfloat16().float() * w[t, j].float()[:, None])
+    return y
+
+
+@pytest.mark.parametrize("T,E,hot", [(1, 512, False), (3, 8, False), (47, 64, False), (130, 4, False), (130, 16, True), (257, 8, True)])
+def test_expert_products_touch_live_rows_only(K, T, E, hot):
+    """FP8 experts with no, one, a few and more than a tile of rows each, against an oracle that rounds where the kernels do.  What is
+    left: rows rounded to bf16 (2^-9), and where another order of the sums turns a group's largest bf16 value, a scale that is
+    2^-8 off, which moves up to one in 16 of the group's values to the next FP8 number (a step of 2^-3 to 2^-4): sqrt(1 / 16) * 0.09
+    = 0.02 of that row."""
+    torch.manual_seed(T + E)
+    H, I, k = 256, 128, 3
+    ex = ExpertWeights.from_dense((torch.randn(E, 2 * I, H, device=DEV) * 0.05).bfloat16(), (torch.randn(E, H, I, device=DEV) * 0.05).bfloat16(),
+                                  "fp8_block")
+    logits = torch.randn(T, E, device=DEV)
+    if hot:
+        logits[:, 1] += 20.0                       # one expert gets every token: full tiles and a remainder
+    w, ids = ref.moe_route(logits, k, True)
+    x = torch.randn(T, H, device=DEV).bfloat16()
+    got = K.moe_forward(x, w.contiguous(), ids.contiguous(), ex, 0, None, "auto")
+    assert K.check_status() == 0
+    assert _rel(got, _fp8_experts(x, ex, w, ids, 0)) < 0.02
+    # a slice of the experts: pairs of the others take no row
+    lo, n = E // 4, E // 2
+    part = ExpertWeights("fp8_block", ex.w13[lo:lo + n].contiguous(), ex.w2[lo:lo + n].contiguous(), ex.w13_scale[lo:lo + n].contiguous(),
+                         ex.w2_scale[lo:lo + n].contiguous())
+    got = K.moe_forward(x, w.contiguous(), ids.contiguous(), part, lo, None, "auto")
+    want = _fp8_experts(x, part, w, ids, lo)
+    assert _rel(got, want) < 0.02 if float(want.abs().max()) > 0 else float(got.abs().max()) == 0
+
+
+def test_expert_row_lists(K):
+    """align: every routed pair has a row of its own inside its expert's segment, and the tiles say how many rows live."""
+    torch.manual_seed(0)
+    T, k, E, lo, n = 75, 4, 32, 8, 16
+    ids = torch.stack([torch.randperm(E)[:k] for _ in range(T)]).int().to(DEV)
+    tiles = T * k // 128 + min(T * k, n)
+    slot, rows = torch.empty(T * k, dtype=torch.int32, device=DEV), torch.full((tiles * 128,), -7, dtype=torch.int32, device=DEV)
+    te, tr, nt = (torch.zeros(m, dtype=torch.int32, device=DEV) for m in (tiles, tiles, 1))
+    K._check(K.lib().atlas_moe_align(ids.data_ptr(), T, k, lo, n, slot.data_ptr(), rows.data_ptr(), te.data_ptr(), tr.data_ptr(), nt.data_ptr(),
+                                     tiles * 128, K._status_ptr[K._dev(ids)], K._stream()), "moe_align")
+    live = int(nt)
+    assert int(tr[:live].sum()) == int(((ids >= lo) & (ids < lo + n)).sum())
+    flat, slot = ids.flatten().tolist(), slot.tolist()
+    used = [s for s in slot if s >= 0]
+    assert len(set(used)) == len(used)
+    for i, (e, s) in enumerate(zip(flat, slot)):
+        assert (s >= 0) == (lo <= e < lo + n)
+        if s >= 0:
+            assert int(te[s // 128]) == e - lo and s % 128 < int(tr[s // 128]) and int(rows[s]) == i // k
+    for t in range(live):
+        assert (rows[t * 128 + int(tr[t]):(t + 1) * 128] == -1).all()
+
+
+# ----------------------------------------------------------------------------- decode graphs of Gated DeltaNet models
+@pytest.mark.parametrize("n", [1, 3, 9])
+def test_delta_net_decode_graph_equals_eager_steps(K, n):
+    """Three decode steps from the same states, replayed and eager (padding rows included): the same bits."""
+    cfg = PRESETS["tiny-hybrid"]("bfloat16")
+    model = build_model(cfg, device=DEV, with_mtp=False).init_random(0, max_pos=256)
+    outs = []
+    for graphs in (True, False):
+        eng = LLMEngine(model, EngineConfig(max_seq_len=256, num_kv_blocks=64, max_num_seqs=n, max_batch_size=n, use_cuda_graphs=graphs,
+                                            enable_prefix_caching=False))
+        gen = torch.Generator(device=DEV).manual_seed(5)
+        for i, st in eng.cache.states.items():
+            st["h"][:n] = torch.randn(st["h"][:n].shape, generator=gen, device=DEV) * 0.1
+            st["conv"][:n] = torch.randn(st["conv"][:n].shape, generator=gen, device=DEV).bfloat16()
+        for k, v in eng.cache.kv.values():
+            k.copy_(torch.zeros(k.shape, device=DEV).to(k.dtype))
+            v.copy_(torch.zeros(v.shape, device=DEV).to(v.dtype))
+        got = []
+        for s in range(3):
+            b = ForwardBatch.build([[7 * i + s + 1] for i in range(n)], [4 + s] * n, [[2 * i, 2 * i + 1] for i in range(n)], 16, device=DEV,
+                                   state_slots=list(range(n)), has_state=[True] * n)
+            with torch.inference_mode():
+                got.append(eng.runner.forward(b).clone())
+        assert (eng.runner.graph_replays == 3) == graphs
+        outs.append(got + [st["h"][:n].clone() for st in eng.cache.states.values()] + [st["conv"][:n].clone() for st in eng.cache.states.values()])
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
