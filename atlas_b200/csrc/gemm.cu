@@ -459,8 +459,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                      &sc_full[sc_slot]);
             if (++sc_slot == kScaleSlots) sc_slot = 0;
           }
-          for (int r = 0; r < a_rows; r += p.a_box_rows)
-            tma_load_2d(sa + r * kRowBytes, &tmap_a, &full[stage], kb * kElemsPerRow, m_tile * kBlockM + r);
+          tma_load_2d(sa, &tmap_a, &full[stage], kb * kElemsPerRow, m_tile * kBlockM);
+          if (p.tile_rows)
+            for (int r = p.a_box_rows; r < a_rows; r += p.a_box_rows)
+              tma_load_2d(sa + r * kRowBytes, &tmap_a, &full[stage], kb * kElemsPerRow, m_tile * kBlockM + r);
           if (p.epi_mode == 1) {
             // 32-row chunks, gate and up alternating, so that an epilogue thread's 64 columns are 32 gate values and
             // the 32 up values of the same activation columns (the tensor map of B has a 32-row box in this mode)
