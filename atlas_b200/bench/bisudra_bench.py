@@ -95,7 +95,7 @@ def kernel_table(size: str, timer, peaks) -> List[dict]:
 
         def plain_conv():
             K._check(R._lib().atlas_conv1d_bias_silu(y.data_ptr(), W, conv.w.data_ptr(), None, W, TAPS, win.data_ptr(), meta.seq_of.data_ptr(), meta.qsl.data_ptr(),
-                                                     meta.slots.data_ptr(), meta.has.data_ptr(), out.data_ptr(), W, T, 1, 0, K._stream()), "conv1d")
+                                                     meta.slots.data_ptr(), meta.has.data_ptr(), out.data_ptr(), W, T, 1, 0, 0, K._stream()), "conv1d")
             R._input_conv_state(conv, y, meta, win)
         add("convolution", "conv1d, silu, window (existing)", shape, plain_conv, T * W * 4 + nseq * W * (TAPS - 1) * 4)
         # ---- products

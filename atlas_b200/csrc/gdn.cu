@@ -1,7 +1,4 @@
-// Gated DeltaNet kernels (Qwen3-Next linear attention), varlen over the step's sequences:
-//   gdn_conv_kernel        depthwise causal conv1d (width W <= 8) + SiLU over the mixed q|k|v channels, reading the
-//                          per-sequence conv window from the state slot
-//   gdn_conv_state_kernel  rolls the conv window forward (optionally only the first `limit` rows: write-on-accept)
+// Gated DeltaNet kernels (Qwen3-Next linear attention), varlen over the step's sequences (the convolution in front: conv1d.cu):
 //   gdn_recurrent_kernel   h_t = exp(g_t) h_{t-1} + k_t (x) ((v_t - h_{t-1}^T k_t) beta_t),  o_t = h_t^T q_t / sqrt(Dk)
 //                          one CTA per (value head, sequence); thread j keeps column j of the fp32 state in registers;
 //                          q/k L2-normalisation and the gates (g from A_log / dt_bias, beta = sigmoid(b)) are fused in.
@@ -9,72 +6,11 @@
 //                          write-on-accept fold (commit with a row limit) and prefill chunks, and can store
 //                          mid-chunk snapshots of the state for the prefix cache.
 // State layout: h [slots, Hv, Dk, Dv] fp32, conv window [slots, C, W-1] bf16.
-// Reference ops replaced: kernels/gb10/common/{causal_conv1d,ssm_preprocess,gated_delta_rule*}.cu.
+// Reference ops replaced: kernels/gb10/common/{ssm_preprocess,gated_delta_rule*}.cu.
 #include "common.cuh"
 #include "host_api.h"
 
 namespace atlas {
-
-__global__ void __launch_bounds__(256)
-gdn_conv_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ w, int C, int W,
-                const __nv_bfloat16* __restrict__ conv_state, const int* __restrict__ seq_of_token,
-                const int* __restrict__ query_start_loc, const int* __restrict__ state_slots,
-                const unsigned char* __restrict__ has_state, __nv_bfloat16* y, long long ldy, int T) {
-  const int t = blockIdx.x;           // rows on grid.x (no 65535 limit)
-  const int c = blockIdx.y * blockDim.x + threadIdx.x;
-  if (c >= C || t >= T) return;
-  const int b = seq_of_token[t];
-  const int q0 = query_start_loc[b];
-  const int rel = t - q0;                      // row inside this sequence's chunk
-  const long long slot = state_slots[b];
-  const bool live = has_state[b] != 0;
-  float acc = 0.f;
-  // tap i multiplies the input i - (W-1) rows back... weight[c][W-1] is the current row
-  for (int i = 0; i < W; ++i) {
-    const int back = W - 1 - i;                // rows back from t
-    float xv;
-    if (back <= rel) {
-      xv = __bfloat162float(x[(long long)(t - back) * ldx + c]);
-    } else {
-      const int sidx = (W - 1) - (back - rel);  // position in the stored window (oldest first)
-      xv = live ? __bfloat162float(conv_state[(slot * C + c) * (W - 1) + sidx]) : 0.f;
-    }
-    acc += xv * __bfloat162float(w[c * W + i]);
-  }
-  y[(long long)t * ldy + c] = __float2bfloat16_rn(acc / (1.f + __expf(-acc)));
-}
-
-// new window = last W-1 entries of (old window ++ first n rows of the chunk), n = limit ? limit[b] : q_len
-__global__ void __launch_bounds__(256)
-gdn_conv_state_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, int C, int W, __nv_bfloat16* conv_state,
-                      const int* __restrict__ query_start_loc, const int* __restrict__ state_slots,
-                      const unsigned char* __restrict__ has_state, const int* __restrict__ limit,
-                      const int* __restrict__ snap_rows, const int* __restrict__ snap_slots, int num_snaps_per_seq) {
-  const int b = blockIdx.y;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  const int q0 = query_start_loc[b];
-  const int qlen = query_start_loc[b + 1] - q0;
-  const long long slot = state_slots[b];
-  const bool live = has_state[b] != 0;
-  float old[8];
-  for (int i = 0; i < W - 1; ++i) old[i] = live ? __bfloat162float(conv_state[(slot * C + c) * (W - 1) + i]) : 0.f;
-  auto window_after = [&](int n, long long dst_slot) {
-    for (int i = 0; i < W - 1; ++i) {
-      const int src = n - (W - 1) + i;          // index into the chunk rows; negative -> old window
-      float v;
-      if (src >= 0) v = __bfloat162float(x[(long long)(q0 + src) * ldx + c]);
-      else v = old[(W - 1) + src];
-      conv_state[(dst_slot * C + c) * (W - 1) + i] = __float2bfloat16_rn(v);
-    }
-  };
-  for (int s = 0; s < num_snaps_per_seq; ++s) {
-    const int rows = snap_rows[b * num_snaps_per_seq + s];
-    if (rows > 0 && rows <= qlen) window_after(rows, snap_slots[b * num_snaps_per_seq + s]);
-  }
-  const int n = limit ? limit[b] : qlen;
-  if (n >= 0 && !(limit && n == 0)) window_after(n, slot);
-}
 
 struct GdnParams {
   const __nv_bfloat16* y; long long ldy;      // conv output: [T, 2*Hk*Dk + Hv*Dv] = q | k | v
@@ -382,31 +318,6 @@ gdn_chunk_kernel(const GdnParams p) {
 }  // namespace atlas
 
 using namespace atlas;
-
-extern "C" int atlas_gdn_conv(const void* x, long long ldx, const void* w, int C, int W, const void* conv_state,
-                              const int* seq_of_token, const int* query_start_loc, const int* state_slots,
-                              const unsigned char* has_state, void* y, long long ldy, int T, void* stream) {
-  if (T <= 0) return 0;
-  if (W < 2 || W > 8) return -1;
-  dim3 grid(T, (C + 255) / 256);
-  gdn_conv_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), ldx, reinterpret_cast<const __nv_bfloat16*>(w), C, W,
-      reinterpret_cast<const __nv_bfloat16*>(conv_state), seq_of_token, query_start_loc, state_slots, has_state,
-      reinterpret_cast<__nv_bfloat16*>(y), ldy, T);
-  return cudaGetLastError() == cudaSuccess ? 0 : -20;
-}
-
-extern "C" int atlas_gdn_conv_state(const void* x, long long ldx, int C, int W, void* conv_state,
-                                    const int* query_start_loc, const int* state_slots, const unsigned char* has_state,
-                                    const int* limit, const int* snap_rows, const int* snap_slots, int num_snaps_per_seq,
-                                    int B, void* stream) {
-  if (B <= 0) return 0;
-  dim3 grid((C + 255) / 256, B);
-  gdn_conv_state_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), ldx, C, W, reinterpret_cast<__nv_bfloat16*>(conv_state), query_start_loc,
-      state_slots, has_state, limit, snap_rows, snap_slots, num_snaps_per_seq);
-  return cudaGetLastError() == cudaSuccess ? 0 : -20;
-}
 
 extern "C" int atlas_gdn_recurrent(const void* y, long long ldy, const void* a, long long lda, const void* b, long long ldb,
                                    const float* A_log, const float* dt_bias, float* h, void* out, long long ldo,

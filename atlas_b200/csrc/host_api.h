@@ -101,12 +101,6 @@ int atlas_moe_plain_combine(const void* y, long long ldy, const int* slot_of, co
                             long long ldo, int f32, void* stream);
 
 // ---- Gated DeltaNet (gdn.cu)
-int atlas_gdn_conv(const void* x, long long ldx, const void* w, int C, int W, const void* conv_state,
-                   const int* seq_of_token, const int* query_start_loc, const int* state_slots,
-                   const unsigned char* has_state, void* y, long long ldy, int T, void* stream);
-int atlas_gdn_conv_state(const void* x, long long ldx, int C, int W, void* conv_state, const int* query_start_loc,
-                         const int* state_slots, const unsigned char* has_state, const int* limit, const int* snap_rows,
-                         const int* snap_slots, int num_snaps_per_seq, int B, void* stream);
 int atlas_gdn_recurrent(const void* y, long long ldy, const void* a, long long lda, const void* b, long long ldb,
                         const float* A_log, const float* dt_bias, float* h, void* out, long long ldo,
                         const int* query_start_loc, const int* state_slots, const unsigned char* has_state,
@@ -266,9 +260,9 @@ int atlas_map_difference(const void* a, const void* gate, long long ldg, void* o
                          int f32, void* stream);
 
 // ---- short convolution (conv1d.cu)
-int atlas_conv1d_bias_silu(const void* x, long long ldx, const void* w, const void* bias, int C, int W, const void* state,
+int atlas_conv1d_bias_silu(const void* x, long long ldx, const void* w, const void* bias, int C, int W, void* state,
                            const int* seq_of_token, const int* qsl, const int* slots, const unsigned char* has, void* y, long long ldy,
-                           int rows, int silu, int f32, void* stream);
+                           int rows, int silu, int advance, int f32, void* stream);
 int atlas_conv1d_add(const void* x, long long ldx, const void* w, int C, int W, void* state, const int* seq_of_token, const int* qsl,
                      const int* slots, const unsigned char* has, void* y, long long ldy, int rows, int advance, int f32, void* stream);
 int atlas_conv1d_state(const void* x, long long ldx, int C, int W, void* state, const int* qsl, const int* slots,

@@ -18,8 +18,6 @@ def _lib():
     global _bound
     lib = K.lib()
     if not _bound:
-        lib.atlas_gdn_conv.argtypes = [_vp, _ll, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _i, _vp]
-        lib.atlas_gdn_conv_state.argtypes = [_vp, _ll, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp]
         lib.atlas_gdn_recurrent.argtypes = [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp,
                                             _vp, _i, _i, _i, _i, _i, _i, _i, _vp]
         lib.atlas_gdn_chunked.argtypes = [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _i,
@@ -76,6 +74,7 @@ class _Meta:
 
 
 def _run(layer, mixed, a, b, meta: _Meta, state, commit: bool):
+    from . import cuda_recurrent
     lib, st = _lib(), K._stream()
     K._dev(mixed)
     T, Cc = mixed.shape
@@ -84,9 +83,7 @@ def _run(layer, mixed, a, b, meta: _Meta, state, commit: bool):
     conv, h = state["conv"], state["h"]
     assert conv.dtype == torch.bfloat16 and h.dtype == torch.float32 and conv.is_contiguous() and h.is_contiguous()
     cw = layer.conv_w if layer.conv_w.dtype == torch.bfloat16 else layer.conv_w.bfloat16()
-    K._check(lib.atlas_gdn_conv(mixed.data_ptr(), mixed.stride(0), cw.data_ptr(), Cc, layer.W, conv.data_ptr(),
-                                meta.seq_of.data_ptr(), meta.qsl.data_ptr(), meta.slots.data_ptr(), meta.has.data_ptr(),
-                                y.data_ptr(), Cc, T, st), "gdn_conv")
+    cuda_recurrent.conv_silu(mixed, cw, None, conv, meta, y, commit, silu=2)
     rc = 1
     if USE_CHUNKED and meta.chunk_ok and commit and layer.dk == 128 and layer.dv == 128:
         rc = lib.atlas_gdn_chunked(y.data_ptr(), Cc, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0),
@@ -102,11 +99,7 @@ def _run(layer, mixed, a, b, meta: _Meta, state, commit: bool):
                                        layer.hv * layer.dv, meta.qsl.data_ptr(), meta.slots.data_ptr(), meta.has.data_ptr(),
                                        K._ptr(meta.limit), meta.snap_rows.data_ptr(), meta.snap_slots.data_ptr(), meta.snaps,
                                        meta.B, layer.hk, layer.hv, layer.dk, layer.dv, 1 if commit else 0, st), "gdn_recurrent")
-    if commit:
-        K._check(lib.atlas_gdn_conv_state(mixed.data_ptr(), mixed.stride(0), Cc, layer.W, conv.data_ptr(), meta.qsl.data_ptr(),
-                                          meta.slots.data_ptr(), meta.has.data_ptr(), K._ptr(meta.limit),
-                                          meta.snap_rows.data_ptr(), meta.snap_slots.data_ptr(), meta.snaps, meta.B, st),
-                 "gdn_conv_state")
+    cuda_recurrent.conv_advance(mixed, layer.W, conv, meta, commit)
     return out
 
 

@@ -50,7 +50,7 @@ def _lib():
         lib.atlas_mlstm_gates.argtypes = [_vp, _ll, _vp, _f] + [_vp] * 10 + [_i] * 4 + [_vp]
         lib.atlas_mlstm_scan.argtypes = [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _vp, _vp, _f, _vp, _vp, _ll] + [_vp] * 7 + [_i] * 8 + [_vp]
         lib.atlas_mlstm_chunk.argtypes = [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _vp, _vp, _f, _vp, _vp, _ll] + [_vp] * 6 + [_i] * 6 + [_vp]
-        lib.atlas_conv1d_bias_silu.argtypes = [_vp, _ll, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _i, _i, _i, _vp]
+        lib.atlas_conv1d_bias_silu.argtypes = [_vp, _ll, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _i, _i, _i, _i, _vp]
         lib.atlas_conv1d_state.argtypes = [_vp, _ll, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp]
         lib.atlas_rope_kv_write_f32.argtypes = [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _i, _i, _f, _vp]
         lib.atlas_attn_f32.argtypes = [_vp, _ll, _vp, _ll, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _f, _i, _i, _i, _i, _i, _i, _vp, _f, _vp, _i, _vp]
@@ -140,6 +140,22 @@ def group_norm_gate(y, z, w, group: int, eps: float, gate_first: bool, gate: str
     return out
 
 
+def conv_silu(x, w, bias, state, meta: _Meta, y, commit: bool, silu: int = 1) -> None:
+    """``y = silu(conv(x) + bias)`` of a recurrent mixer's input; steps of one row per sequence move their windows on in the same launch."""
+    K._check(_lib().atlas_conv1d_bias_silu(x.data_ptr(), x.stride(0), w.data_ptr(), K._ptr(bias), x.shape[1], w.shape[1], state.data_ptr(),
+                                           meta.seq_of.data_ptr(), meta.qsl.data_ptr(), meta.slots.data_ptr(), meta.has.data_ptr(),
+                                           y.data_ptr(), y.stride(0), x.shape[0], silu, 1 if commit and meta.one_row else 0, _f32(x),
+                                           K._stream()), "conv1d")
+
+
+def conv_advance(x, taps: int, state, meta: _Meta, commit: bool) -> None:
+    """The windows after a committed step, where :func:`conv_silu` has not written them."""
+    if commit and not meta.one_row:
+        K._check(_lib().atlas_conv1d_state(x.data_ptr(), x.stride(0), x.shape[1], taps, state.data_ptr(), meta.qsl.data_ptr(),
+                                           meta.slots.data_ptr(), meta.has.data_ptr(), K._ptr(meta.limit), meta.snap_rows.data_ptr(),
+                                           meta.snap_slots.data_ptr(), meta.snaps, meta.B, _f32(x), K._stream()), "conv1d_state")
+
+
 def _mamba2_run(layer, xbc, dt, meta: _Meta, state, commit: bool):
     lib, st = _lib(), K._stream()
     K._dev(xbc)
@@ -151,19 +167,13 @@ def _mamba2_run(layer, xbc, dt, meta: _Meta, state, commit: bool):
     assert layer.conv_b is None or layer.conv_b.dtype == xbc.dtype
     y = torch.empty(T, Cc, dtype=xbc.dtype, device=xbc.device)
     out = torch.empty(T, layer.d_inner, dtype=xbc.dtype, device=xbc.device)
-    K._check(lib.atlas_conv1d_bias_silu(xbc.data_ptr(), xbc.stride(0), layer.conv_w.data_ptr(), K._ptr(layer.conv_b), Cc, layer.W,
-                                        conv.data_ptr(), meta.seq_of.data_ptr(), meta.qsl.data_ptr(), meta.slots.data_ptr(),
-                                        meta.has.data_ptr(), y.data_ptr(), Cc, T, 1, f32, st), "conv1d")
+    conv_silu(xbc, layer.conv_w, layer.conv_b, conv, meta, y, commit)
     K._check(lib.atlas_mamba2_scan(y.data_ptr(), Cc, dt.data_ptr(), dt.stride(0), layer.A_log.data_ptr(), layer.D.data_ptr(),
                                    layer.dt_bias.data_ptr(), float(layer.cfg.mamba_dt_min), h.data_ptr(), out.data_ptr(),
                                    layer.d_inner, meta.qsl.data_ptr(), meta.slots.data_ptr(), meta.has.data_ptr(),
                                    K._ptr(meta.limit), meta.snap_rows.data_ptr(), meta.snap_slots.data_ptr(), meta.snaps, meta.B,
                                    layer.h, layer.p, layer.n, layer.g, 1 if commit else 0, meta.one_row, f32, st), "mamba2_scan")
-    if commit:
-        K._check(lib.atlas_conv1d_state(xbc.data_ptr(), xbc.stride(0), Cc, layer.W, conv.data_ptr(), meta.qsl.data_ptr(),
-                                        meta.slots.data_ptr(), meta.has.data_ptr(), K._ptr(meta.limit),
-                                        meta.snap_rows.data_ptr(), meta.snap_slots.data_ptr(), meta.snaps, meta.B, f32, st),
-                 "conv1d_state")
+    conv_advance(xbc, layer.W, conv, meta, commit)
     return out
 
 
@@ -289,7 +299,7 @@ def _rglru_run(layer, y, x, meta: _Meta, state, commit: bool):
         u = torch.empty(T, Cc, dtype=x.dtype, device=x.device)
         K._check(lib.atlas_conv1d_bias_silu(x.data_ptr(), x.stride(0), layer.conv_w.data_ptr(), layer.conv_b.data_ptr(), Cc, layer.W, conv.data_ptr(),
                                             meta.seq_of.data_ptr(), meta.qsl.data_ptr(), meta.slots.data_ptr(), meta.has.data_ptr(), u.data_ptr(),
-                                            Cc, T, 0, f32, st), "conv1d")
+                                            Cc, T, 0, 0, f32, st), "conv1d")
         # gate sums [2, blocks, T, n] in fp32
         z = torch.matmul(u.float().view(T, layer.blocks, layer.n).transpose(0, 1), layer.gates.float().transpose(2, 3))
         a.u, a.ldu, a.zr, a.zi, a.z_row, a.z_block = u.data_ptr(), Cc, z[0].data_ptr(), z[1].data_ptr(), layer.n, T * layer.n
