@@ -1,5 +1,5 @@
-// Prefill (chunk) attention over the paged FP8 KV cache on the 5th-generation tensor cores (head_dim 128, 16-token
-// pages).  One CTA per (128-row query tile, kv head); the G = Hq/Hkv query heads that share the kv head are packed into
+// Prefill (chunk) attention over the paged FP8 KV cache on the 5th-generation tensor cores (head_dim 128 or 256,
+// 16-token pages).  One CTA per (128-row query tile, kv head); the G = Hq/Hkv query heads that share the kv head are packed into
 // the tile's rows (row = token * G + head), so every K/V page is fetched and widened once for all of them.
 //
 //   warp 0       producer: TMA load of the Q tile (3-D box: 64 dims x G heads x 128/G tokens, 128-byte swizzle) and
@@ -19,6 +19,9 @@
 // scale is applied with the final 1/l.  QK_{j+1} is issued before PV_j, so the tensor cores work on the next score tile
 // while the softmax warps handle the current one.  Every wait is bounded (status word + early exit).
 //
+// Bound at head dim 256 by shared memory: per 64 keys the products read 144 KB and the converters move 96 KB.  One 8192-token prompt, 16
+// query heads on 2 kv heads: 4690 us with the general mma.sync kernel, 1014 us; 517 rows behind 4096 cached ones 759 to 172 us.
+//
 // Reference ops replaced: inferspark_prefill_paged_fp8.cu / prefill_paged_compute.cuh (mma.sync FA2, QK^T in bf16 and
 // P.V in fp16) and the FlashInfer ragged-prefill wrapper.
 #include <mutex>
@@ -30,16 +33,23 @@
 
 namespace atlas {
 
-constexpr int kTcD = 128;                 // head dim
 constexpr int kTcRows = 128;              // query rows per tile (tokens * G)
-constexpr int kTcKv = 128;                // kv tokens per tile
 constexpr int kTcPage = 16;
-constexpr int kTcPages = kTcKv / kTcPage;
 constexpr int kTcThreads = 448;
 constexpr int kSub = 16 * 1024;           // one 128-row x 64-element f16 sub-tile
-constexpr int kPageBytes = kTcPage * kTcD;        // 2 KB (fp8)
-constexpr int kStageBytes = 2 * kTcPages * kPageBytes;   // K pages then V pages: 32 KB
-constexpr int kTcStages = 3;
+// Head dim 128 works on KV tiles of 128 tokens and stages three of them.  Head dim 256 on 64 tokens and two stages: Q (64 KB), the
+// widened K and V (32 KB each), P and the staged pages then take 208 KB of shared memory; 128 tokens would need more than there is.
+template <int D>
+struct TcTile {
+  static constexpr int kKv = D == 128 ? 128 : 64;                // kv tokens per tile
+  static constexpr int kPages = kKv / kTcPage;
+  static constexpr int kKSub = kKv * 128, kVSub = D * 128;       // 64-element wide f16 sub-tiles of K (rows: tokens) and V (rows: dims)
+  static constexpr int kPageBytes = kTcPage * D;                 // fp8
+  static constexpr int kStageBytes = 2 * kPages * kPageBytes;    // K pages then V pages: 32 KB
+  static constexpr int kStages = D == 128 ? 3 : 2;
+  static constexpr int kTiles = (D / 64) * (kSub + kKSub) + (kKv / 64) * (kVSub + kSub);
+  static constexpr int kSmem = kTiles + kStages * kStageBytes + 256 + 1024;
+};
 
 struct TcAttnParams {
   __nv_bfloat16* out; long long ldo;
@@ -79,15 +89,19 @@ ATLAS_DEVICE void widen16(const uint4 v, uint4& lo, uint4& hi) {
 }
 
 // 14 warps are accounted as 16 (warps are allocated four at a time), so 128 registers per thread is the ceiling
+template <int D>
 __global__ void __launch_bounds__(kTcThreads, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = smem;                       // 2 sub-tiles: [128 rows][64 dims]
-  uint8_t* sK = smem + 2 * kSub;            // 2 sub-tiles: [128 tokens][64 dims]
-  uint8_t* sV = smem + 4 * kSub;            // 2 sub-tiles: [128 dims][64 tokens]
-  uint8_t* sP = smem + 6 * kSub;            // 2 sub-tiles: [128 rows][64 tokens]
-  uint8_t* sStage = smem + 8 * kSub;        // kTcStages x (8 K pages + 8 V pages)
+  using Tile = TcTile<D>;
+  constexpr int kTcKv = Tile::kKv, kTcPages = Tile::kPages, kTcStages = Tile::kStages, kStageBytes = Tile::kStageBytes;
+  constexpr int kPageBytes = Tile::kPageBytes, kKSub = Tile::kKSub, kVSub = Tile::kVSub;
+  uint8_t* sQ = smem;                       // D / 64 sub-tiles: [128 rows][64 dims]
+  uint8_t* sK = sQ + (D / 64) * kSub;       // D / 64 sub-tiles: [tokens][64 dims]
+  uint8_t* sV = sK + (D / 64) * kKSub;      // kTcKv / 64 sub-tiles: [dims][64 tokens]
+  uint8_t* sP = sV + (kTcKv / 64) * kVSub;  // kTcKv / 64 sub-tiles: [128 rows][64 tokens]
+  uint8_t* sStage = smem + Tile::kTiles;    // kTcStages x (K pages, V pages)
   uint64_t* bars = reinterpret_cast<uint64_t*>(sStage + kTcStages * kStageBytes);
   uint64_t* q_full = bars;                  // 1
   uint64_t* stg_full = bars + 1;            // [kTcStages] tx
@@ -134,20 +148,20 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tS = tmem_base;            // two score buffers: columns [0,128) and [128,256)
-  const uint32_t tO = tmem_base + 256;      // output accumulator: columns [256,384)
-  const uint32_t tX = tmem_base + 384;      // four columns through which the two threads of a row exchange a value
+  const uint32_t tS = tmem_base;            // two score buffers of kTcKv columns
+  const uint32_t tO = tmem_base + 2 * kTcKv;          // output accumulator: D columns
+  const uint32_t tX = tmem_base + 2 * kTcKv + D;      // four columns through which the two threads of a row exchange a value
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer (whole warp)
     if (lane == 0) {
-      mbar_expect_tx(q_full, 2 * kSub);
-      tma_load_3d(sQ, &tmap_q, q_full, 0, kvh * G, q_row0 + q0);
-      tma_load_3d(sQ + kSub, &tmap_q, q_full, 64, kvh * G, q_row0 + q0);
+      mbar_expect_tx(q_full, (D / 64) * kSub);
+#pragma unroll
+      for (int s = 0; s < D / 64; ++s) tma_load_3d(sQ + s * kSub, &tmap_q, q_full, s * 64, kvh * G, q_row0 + q0);
     }
     const int* bt = p.block_tables + (long long)b * p.bt_ld;
     const int n_pages = (L + kTcPage - 1) / kTcPage;
-    const int pi = lane & 7;                          // lanes 0..7 copy K pages, 8..15 V pages
+    const int pi = lane & 7;                          // lanes 0..7 copy K pages, 8..15 V pages (the first kTcPages of them)
     int blk_next = (lane < 16 && pi < n_pages) ? bt[pi] : 0;
     uint32_t stage = 0, phase = 0;
     bool ok = true;
@@ -174,7 +188,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0) {
-      constexpr uint32_t kIdesc = make_idesc(kTcRows, 128, 0u);       // f16 x f16 -> f32, M = 128, N = 128
+      constexpr uint32_t kIdescS = make_idesc(kTcRows, kTcKv, 0u), kIdescO = make_idesc(kTcRows, D, 0u);     // f16 x f16 -> f32
       const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK), aV = smem_u32(sV), aP = smem_u32(sP);
       bool ok = mbar_wait(q_full, 0, abort_flag, p.status, 0x810) && mbar_wait(q_conv, 0, abort_flag, p.status, 0x811);
       auto issue_pv = [&](int i) -> bool {
@@ -182,10 +196,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
         if (!mbar_wait(v_ready, i & 1, abort_flag, p.status, 0x813)) return false;
         tc_fence_after();
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
+        for (int ks = 0; ks < kTcKv / 16; ++ks) {
           const uint64_t ad = make_smem_desc_sw128(aP + (ks >> 2) * kSub) + 2 * (ks & 3);
-          const uint64_t bd = make_smem_desc_sw128(aV + (ks >> 2) * kSub) + 2 * (ks & 3);
-          umma_f16(tO, ad, bd, kIdesc, (i > 0 || ks > 0) ? 1u : 0u);
+          const uint64_t bd = make_smem_desc_sw128(aV + (ks >> 2) * kVSub) + 2 * (ks & 3);
+          umma_f16(tO, ad, bd, kIdescO, (i > 0 || ks > 0) ? 1u : 0u);
         }
         umma_commit(pv_done);
         return true;
@@ -196,10 +210,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
         if (!mbar_wait(&s_free[sb], ((j >> 1) & 1) ^ 1u, abort_flag, p.status, 0x815)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
+        for (int ks = 0; ks < D / 16; ++ks) {
           const uint64_t ad = make_smem_desc_sw128(aQ + (ks >> 2) * kSub) + 2 * (ks & 3);
-          const uint64_t bd = make_smem_desc_sw128(aK + (ks >> 2) * kSub) + 2 * (ks & 3);
-          umma_f16(tS + sb * 128, ad, bd, kIdesc, ks > 0 ? 1u : 0u);
+          const uint64_t bd = make_smem_desc_sw128(aK + (ks >> 2) * kKSub) + 2 * (ks & 3);
+          umma_f16(tS + sb * kTcKv, ad, bd, kIdescS, ks > 0 ? 1u : 0u);
         }
         umma_commit(&s_full[sb]);
         umma_commit(k_free);
@@ -217,7 +231,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
     if (ok) {
       const int t384 = threadIdx.x - 64;                          // 0..383 over both roles
       uint4* q4 = reinterpret_cast<uint4*>(sQ);
-      for (int i = t384; i < 2 * kSub / 16; i += 384) {
+      for (int i = t384; i < (D / 64) * kSub / 16; i += 384) {
         uint4 v = q4[i];
         uint32_t* w = reinterpret_cast<uint32_t*>(&v);
 #pragma unroll
@@ -234,7 +248,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
 
     if (is_conv) {
       const int r = t128;                    // K: token row of the tile; V: head-dim row
-      const int sw = r & 7;
       // K_{j+1} is converted before V_j: the next score tile can then be issued while the softmax warps are still
       // working on the current one (V_j has to wait for the previous PV product anyway).
       auto conv_k = [&](int j) -> bool {
@@ -243,15 +256,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
         if (j > 0 && !mbar_wait(k_free, (j - 1) & 1, abort_flag, p.status, 0x822)) return false;
         const int kv0 = j * kTcKv;
         // consecutive threads take consecutive 16-byte pieces of the staged pages (no bank conflicts on the read):
-        // piece i = row (token) i / 8, dims (i % 8) * 16 .. + 15
+        // piece i = row (token) i / (D / 16), dims (i % (D / 16)) * 16 .. + 15
         const uint4* src = reinterpret_cast<const uint4*>(sStage + s * kStageBytes);
 #pragma unroll
-        for (int k8 = 0; k8 < 8; ++k8) {
+        for (int k8 = 0; k8 < kTcKv * (D / 16) / 128; ++k8) {
           const int i = k8 * 128 + r;
-          const int trow = i >> 3, c = i & 7, tsw = trow & 7;
+          const int trow = i / (D / 16), c = i % (D / 16), tsw = trow & 7;
           uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
           if (kv0 + trow < L) widen16(src[i], lo, hi);
-          uint8_t* rowp = sK + (c >> 2) * kSub + (trow >> 3) * 1024 + tsw * 128;
+          uint8_t* rowp = sK + (c >> 2) * kKSub + (trow >> 3) * 1024 + tsw * 128;
           const int ch = (c & 3) * 2;
           *reinterpret_cast<uint4*>(rowp + ((ch ^ tsw) << 4)) = lo;
           *reinterpret_cast<uint4*>(rowp + (((ch + 1) ^ tsw) << 4)) = hi;
@@ -265,15 +278,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
         const int s = j % kTcStages;
         const int kv0 = j * kTcKv;
         const uint8_t* stg = sStage + s * kStageBytes;
-        // row r = head dim r, page pg holds tokens kv0 + 16 pg .. + 15 as 16 contiguous bytes
+        // rows r, r + 128 .. = head dims, page pg holds tokens kv0 + 16 pg .. + 15 as 16 contiguous bytes
         if (j > 0 && !mbar_wait(pv_done, (j - 1) & 1, abort_flag, p.status, 0x823)) return false;
-        uint8_t* row0 = sV + (r >> 3) * 1024 + sw * 128;
 #pragma unroll
-        for (int pg = 0; pg < kTcPages; ++pg) {
+        for (int it = 0; it < (D / 128) * kTcPages; ++it) {
+          const int pg = it % kTcPages, dim = r + (it / kTcPages) * 128, sw = dim & 7;
           const int t0 = kv0 + pg * kTcPage;
           uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
           if (t0 < L) {
-            uint4 v = *reinterpret_cast<const uint4*>(stg + (kTcPages + pg) * kPageBytes + r * kTcPage);
+            uint4 v = *reinterpret_cast<const uint4*>(stg + (kTcPages + pg) * kPageBytes + dim * kTcPage);
             if (t0 + kTcPage > L) {                 // the sequence ends inside this page: clear the tail bytes
               uint8_t* bytes = reinterpret_cast<uint8_t*>(&v);
 #pragma unroll
@@ -282,7 +295,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
             }
             widen16(v, lo, hi);
           }
-          uint8_t* rowp = row0 + (pg >> 2) * kSub;
+          uint8_t* rowp = sV + (pg >> 2) * kVSub + (dim >> 3) * 1024 + sw * 128;
           const int ch = (pg & 3) * 2;
           *reinterpret_cast<uint4*>(rowp + ((ch ^ sw) << 4)) = lo;
           *reinterpret_cast<uint4*>(rowp + (((ch + 1) ^ sw) << 4)) = hi;
@@ -300,8 +313,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
     } else {
       // ---------------------------------------------------------------- softmax, two threads per query row
       const int lane_group = warp & 3;                           // the TMEM lanes a warp may touch: 32 * (warp % 4) ..
-      const int half = (warp - 6) >> 2;                          // 0: score / output columns [0, 64), 1: [64, 128)
-      const int col0 = half * 64;
+      const int half = (warp - 6) >> 2;                          // which half of the score and output columns
+      constexpr int HC = kTcKv / 2, HO = D / 2;                   // score and output columns of a thread
+      const int col0 = half * HC, ocol0 = half * HO;
       const int row = lane_group * 32 + lane;
       const uint32_t t_lane = (uint32_t)(lane_group * 32) << 16;
       // One value per thread to the other thread of the same row: written to a TMEM column of the row's lane, handed
@@ -331,27 +345,28 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
       const int pos = ctx0 + tok;                                // absolute position: keys [0, pos] are visible
       float m = -INFINITY, l = 0.f;
       const int sw = row & 7;
-      uint8_t* prow0 = sP + half * kSub + (row >> 3) * 1024 + sw * 128;      // this half's 64 columns are one sub-tile
+      uint8_t* prow0 = sP + (col0 >> 6) * kSub + (row >> 3) * 1024 + sw * 128;
+      const int pch = (col0 >> 3) & 7;                           // this half's first 16-byte chunk in its sub-tile
       for (int j = 0; j < n_kv && ok; ++j) {
         const int sb = j & 1;
         const int kv0 = j * kTcKv;
         if (!mbar_wait(&s_full[sb], (j >> 1) & 1, abort_flag, p.status, 0x830)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t ts = tS + sb * 128 + t_lane;
+        const uint32_t ts = tS + sb * kTcKv + t_lane;
         const int vis = row_live ? min(pos + 1, L) - kv0 : 0;     // columns [0, vis) of this tile are visible to the row
         // ---- this thread's half of the score row into registers, both loads in flight together, then release the buffer
-        uint32_t sr[2][32];
+        uint32_t sr[HC / 32][32];
 #pragma unroll
-        for (int c = 0; c < 2; ++c) tmem_ld_32x32b_x32(ts + col0 + c * 32, sr[c]);
+        for (int c = 0; c < HC / 32; ++c) tmem_ld_32x32b_x32(ts + col0 + c * 32, sr[c]);
         tmem_ld_wait();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&s_free[sb]);
         // tiles below the diagonal need no masking at all (same for every row of the warp)
-        const bool full = __all_sync(0xffffffffu, vis >= col0 + 64);
+        const bool full = __all_sync(0xffffffffu, vis >= col0 + HC);
         if (!full) {
 #pragma unroll
-          for (int c = 0; c < 2; ++c)
+          for (int c = 0; c < HC / 32; ++c)
 #pragma unroll
             for (int i = 0; i < 32; ++i)
               if (col0 + c * 32 + i >= vis) sr[c][i] = 0xff800000u;  // -inf: exp2 gives exactly 0 below
@@ -359,7 +374,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
         // four independent chains (a single running max would serialise 128 dependent instructions)
         float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
+        for (int c = 0; c < HC / 32; ++c)
 #pragma unroll
           for (int i = 0; i < 32; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(sr[c][i]));
         float mx_other;
@@ -378,13 +393,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
           tc_fence_after();
           if (__any_sync(0xffffffffu, alpha != 1.f)) {
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
+            for (int c = 0; c < HO / 32; ++c) {
               uint32_t r[32];
-              tmem_ld_32x32b_x32(tO + t_lane + col0 + c * 32, r);
+              tmem_ld_32x32b_x32(tO + t_lane + ocol0 + c * 32, r);
               tmem_ld_wait();
 #pragma unroll
               for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-              tmem_st_32x32b_x32(tO + t_lane + col0 + c * 32, r);
+              tmem_st_32x32b_x32(tO + t_lane + ocol0 + c * 32, r);
             }
             tmem_st_wait();
           }
@@ -394,7 +409,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
         float sum4[4] = {0.f, 0.f, 0.f, 0.f};
         const float mref = (m_new == -INFINITY) ? 0.f : m_new;       // dead rows: -inf - 0 stays -inf, p = 0
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < HC / 32; ++c) {
           uint8_t* rowp = prow0;
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
@@ -406,7 +421,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
             }
             uint4 o;
             o.x = pack_h2(e[0], e[1]); o.y = pack_h2(e[2], e[3]); o.z = pack_h2(e[4], e[5]); o.w = pack_h2(e[6], e[7]);
-            const int ch = c * 4 + q;
+            const int ch = pch + c * 4 + q;
             *reinterpret_cast<uint4*>(rowp + ((ch ^ sw) << 4)) = o;
           }
         }
@@ -418,19 +433,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
         __syncwarp();
         if (lane == 0) mbar_arrive(p_ready);
       }
-      // ---- epilogue: O / l * v_scale -> bf16, each thread its 64 columns; l is the sum of the two halves' row sums
+      // ---- epilogue: O / l * v_scale -> bf16, each thread its half of the columns; l is the sum of the two halves' row sums
       float l_other = 0.f;
       if (ok && n_kv > 0) ok = exchange(l, l_other);
       l += l_other;
       if (ok && n_kv > 0 && mbar_wait(pv_done, (n_kv - 1) & 1, abort_flag, p.status, 0x832)) {
         tc_fence_after();
         const float inv = (l > 0.f) ? p.v_scale / l : 0.f;
-        if (p.q_out != nullptr) {
+        if (D == 128 && p.q_out != nullptr) {
           // the whole output row in registers (as the score rows were), rounded to bf16 like the unfused path's
           // output, then one scale for the row's 128 values
           uint32_t r[2][32];
 #pragma unroll
-          for (int c = 0; c < 2; ++c) tmem_ld_32x32b_x32(tO + t_lane + col0 + c * 32, r[c]);
+          for (int c = 0; c < 2; ++c) tmem_ld_32x32b_x32(tO + t_lane + ocol0 + c * 32, r[c]);
           tmem_ld_wait();
           float amax = 0.f;
 #pragma unroll
@@ -447,7 +462,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
           if (row_live && got) {
             const float sc = fmaxf(amax, 1e-10f) / 448.f;
             const float qinv = __frcp_rn(sc);
-            uint8_t* qrow = p.q_out + (long long)(q_row0 + tok) * p.ldqo + head * kTcD + col0;
+            uint8_t* qrow = p.q_out + (long long)(q_row0 + tok) * p.ldqo + head * D + ocol0;
 #pragma unroll
             for (int c = 0; c < 2; ++c)
 #pragma unroll
@@ -465,11 +480,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
             if (half == 0) p.s_out[(long long)head * p.s_ld + q_row0 + tok] = sc;
           }
         } else {
-        __nv_bfloat16* orow = p.out + (long long)(q_row0 + tok) * p.ldo + head * kTcD + col0;
+        __nv_bfloat16* orow = p.out + (long long)(q_row0 + tok) * p.ldo + head * D + ocol0;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < HO / 32; ++c) {
           uint32_t r[32];
-          tmem_ld_32x32b_x32(tO + t_lane + col0 + c * 32, r);
+          tmem_ld_32x32b_x32(tO + t_lane + ocol0 + c * 32, r);
           tmem_ld_wait();
           if (row_live) {
 #pragma unroll
@@ -502,7 +517,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcAttnP
 using namespace atlas;
 
 // Chunk attention on tcgen05.  `num_tiles` query tiles of 128/G tokens each, described by (sequence index, first query
-// token of the tile inside the sequence's chunk).  Covers head_dim 128, 16-token pages, an FP8 cache, G = Hq/Hkv in
+// token of the tile inside the sequence's chunk).  Covers head_dim 128 and 256, 16-token pages, an FP8 cache, G = Hq/Hkv in
 // {1,2,4,8} and no sliding window; returns ATLAS_ATTN_TC_UNSUPPORTED (1) otherwise so that the caller can use the
 // general kernel.
 extern "C" int atlas_attn_prefill_tc(const void* q, long long ldq, void* out, long long ldo, const void* k_cache,
@@ -512,8 +527,8 @@ extern "C" int atlas_attn_prefill_tc(const void* q, long long ldq, void* out, lo
                                      int block_size, int window, unsigned long long* status, void* stream, void* q_out,
                                      long long ldqo, float* s_out, long long s_ld) {
   if (num_tiles <= 0) return 0;
-  if (D != kTcD || block_size != kTcPage || window > 0 || Hq % Hkv) return 1;
-  if (q_out != nullptr && (!s_out || (ldqo % 16) || (reinterpret_cast<uintptr_t>(q_out) & 15))) return 1;
+  if ((D != 128 && D != 256) || block_size != kTcPage || window > 0 || Hq % Hkv) return 1;
+  if (q_out != nullptr && (D != 128 || !s_out || (ldqo % 16) || (reinterpret_cast<uintptr_t>(q_out) & 15))) return 1;
   const int G = Hq / Hkv;
   if (G != 1 && G != 2 && G != 4 && G != 8) return 1;
   if ((reinterpret_cast<uintptr_t>(q) & 15) || (ldq * 2) % 16) return 1;
@@ -537,9 +552,11 @@ extern "C" int atlas_attn_prefill_tc(const void* q, long long ldq, void* out, lo
   p.tile_seq = tile_seq; p.tile_q0 = tile_q0;
   p.qk_scale_log2 = scale * k_scale * 1.4426950408889634f; p.v_scale = v_scale;
   p.Hq = Hq; p.Hkv = Hkv; p.G = G; p.total_tokens = total_tokens; p.status = status;
-  constexpr int kSmem = 8 * kSub + kTcStages * kStageBytes + 256 + 1024;
-  if (ensure_dynamic_smem(reinterpret_cast<const void*>(attn_prefill_tc_kernel), kSmem) != cudaSuccess) return -20;
-  dim3 grid(num_tiles, Hkv);
-  attn_prefill_tc_kernel<<<grid, kTcThreads, kSmem, reinterpret_cast<cudaStream_t>(stream)>>>(tq, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  auto launch = [&](auto kern, int smem) {
+    if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) != cudaSuccess) return -20;
+    kern<<<dim3(num_tiles, Hkv), kTcThreads, smem, st>>>(tq, p);
+    return cudaGetLastError() == cudaSuccess ? 0 : -21;
+  };
+  return D == 128 ? launch(attn_prefill_tc_kernel<128>, TcTile<128>::kSmem) : launch(attn_prefill_tc_kernel<256>, TcTile<256>::kSmem);
 }

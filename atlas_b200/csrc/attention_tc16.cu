@@ -1,4 +1,4 @@
-// Prefill (chunk) attention over the paged bf16 KV cache on the 5th-generation tensor cores: head_dim 64 or 128, 16-token
+// Prefill (chunk) attention over the paged bf16 KV cache on the 5th-generation tensor cores: head_dim 64, 128 or 256, 16-token
 // pages, any number of query heads per kv head up to 128, causal with optional chunked visibility, sliding window, softmax
 // sinks, bounded scores and a bias per head by the key's distance.
 //
@@ -8,7 +8,7 @@
 //
 //   warp 0       TMA load of the Q tile (3-D box: 64 dims x G heads x 128/G tokens, 128-byte swizzle)
 //   warp 1       tcgen05.mma issuer (kind::f16 on bf16): S_j = Q K_j^T into one of two TMEM buffers, O += P_j V_j
-//   warps 2, 3   K loaders: cp.async into a ring of two 128-token tiles (rows = tokens)
+//   warps 2, 3   K loaders: cp.async into a ring of two tiles of 128 tokens (64 at head dim 256) (rows = tokens)
 //   warps 4, 5   V loaders: the same for V^T (rows = head dims); pieces past the sequence's end are zeroed
 //   warps 6..13  softmax, two threads per query row (see attention_tc.cu): scores are scaled into the exp2 domain in fp32, P
 //                goes to shared memory in bf16 as the A operand of the PV product, O is rescaled in TMEM lazily
@@ -20,7 +20,9 @@
 
 namespace atlas {
 
-constexpr int kT16Rows = 128, kT16Kv = 128, kT16Page = 16, kT16Pages = kT16Kv / kT16Page, kT16Threads = 448;
+constexpr int kT16Rows = 128, kT16Page = 16, kT16Threads = 448;
+// kv tokens per tile: half as many at head dim 256, so that two K and two V tiles fit beside Q
+constexpr int tc16_kv(int D) { return D == 256 ? 64 : 128; }
 constexpr int kT16Sub = 16 * 1024;            // 128 rows x 64 bf16
 
 struct Tc16Params {
@@ -55,13 +57,15 @@ template <int D>
 __global__ void __launch_bounds__(kT16Threads, 1)
 attn_prefill_tc16_kernel(const __grid_constant__ CUtensorMap tmap_q, const Tc16Params p) {
   constexpr int NS = D / 64;                  // 64-dim sub-tiles of Q and K
+  constexpr int kT16Kv = tc16_kv(D), kT16Pages = kT16Kv / kT16Page;
+  constexpr int kKSub = kT16Kv * 128;         // K sub-tile: 64 dims of every token
   constexpr int kVSub = D * 128;              // V^T sub-tile: D rows x 64 tokens
-  constexpr int kKTile = NS * kT16Sub, kVTile = 2 * kVSub;
+  constexpr int kKTile = NS * kKSub, kVTile = (kT16Kv / 64) * kVSub;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
-  uint8_t* sP = sQ + NS * kT16Sub;            // 2 sub-tiles: [128 rows][64 tokens]
-  uint8_t* sK = sP + 2 * kT16Sub;             // two slots
+  uint8_t* sP = sQ + NS * kT16Sub;            // kT16Kv / 64 sub-tiles: [128 rows][64 tokens]
+  uint8_t* sK = sP + (kT16Kv / 64) * kT16Sub;             // two slots
   uint8_t* sV = sK + 2 * kKTile;              // two slots
   uint64_t* bars = reinterpret_cast<uint64_t*>(sV + 2 * kVTile);
   uint64_t* q_full = bars;
@@ -112,7 +116,7 @@ attn_prefill_tc16_kernel(const __grid_constant__ CUtensorMap tmap_q, const Tc16P
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tS = tmem_base, tO = tmem_base + 256, tX = tmem_base + 384;
+  const uint32_t tS = tmem_base, tO = tmem_base + 2 * kT16Kv, tX = tmem_base + 384;
   const int* bt = p.block_tables + (long long)b * p.bt_ld;
 
   if (warp == 0) {
@@ -150,8 +154,8 @@ attn_prefill_tc16_kernel(const __grid_constant__ CUtensorMap tmap_q, const Tc16P
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks) {
           const uint64_t ad = make_smem_desc_sw128(aQ + (ks >> 2) * kT16Sub) + 2 * (ks & 3);
-          const uint64_t bd = make_smem_desc_sw128(aK + s * kKTile + (ks >> 2) * kT16Sub) + 2 * (ks & 3);
-          umma_f16(tS + s * 128, ad, bd, kIdS, ks > 0 ? 1u : 0u);
+          const uint64_t bd = make_smem_desc_sw128(aK + s * kKTile + (ks >> 2) * kKSub) + 2 * (ks & 3);
+          umma_f16(tS + s * kT16Kv, ad, bd, kIdS, ks > 0 ? 1u : 0u);
         }
         umma_commit(&s_full[s]);
         umma_commit(&k_free[s]);
@@ -178,7 +182,7 @@ attn_prefill_tc16_kernel(const __grid_constant__ CUtensorMap tmap_q, const Tc16P
         for (int it = 0; it < kT16Kv * CPR / 64; ++it) {
           const int i = it * 64 + t, trow = i / CPR, c = i % CPR, pg = trow / kT16Page;
           const long long base = ((long long)__shfl_sync(0xffffffffu, blk, pg) * p.Hkv + kvh) * (kT16Page * D);
-          cp16(dst + (c >> 3) * kT16Sub + (trow >> 3) * 1024 + (trow & 7) * 128 + (((c & 7) ^ (trow & 7)) << 4),
+          cp16(dst + (c >> 3) * kKSub + (trow >> 3) * 1024 + (trow & 7) * 128 + (((c & 7) ^ (trow & 7)) << 4),
                p.k_cache + base + (trow % kT16Page) * D + c * 8, pg0 + pg < n_pages);
         }
       } else {
@@ -216,8 +220,9 @@ attn_prefill_tc16_kernel(const __grid_constant__ CUtensorMap tmap_q, const Tc16P
     if (lane == 0) mbar_arrive(&ready[(n_kv - 1) & 1]);
   } else {
     // ------------------------------------------------------------------ softmax, two threads per query row
-    const int lane_group = warp & 3, half = (warp - 6) >> 2;      // score columns [64 half, + 64), output columns [D/2 half, + D/2)
-    const int col0 = half * 64, ocol0 = half * (D / 2);
+    const int lane_group = warp & 3, half = (warp - 6) >> 2;      // this half of the score and output columns
+    constexpr int HC = kT16Kv / 2;
+    const int col0 = half * HC, ocol0 = half * (D / 2);
     constexpr int OC = D / 64;                                    // 32-column pieces of this thread's output half
     const int row = lane_group * 32 + lane;
     const uint32_t t_lane = (uint32_t)(lane_group * 32) << 16;
@@ -259,37 +264,38 @@ attn_prefill_tc16_kernel(const __grid_constant__ CUtensorMap tmap_q, const Tc16P
     const float bias_far = biased ? bias_row[p.reach] * bias_mul : 0.f;
     float m = -INFINITY, l = 0.f;                                 // m: reference point in the exp2 domain
     const int sw = row & 7;
-    uint8_t* prow = sP + half * kT16Sub + (row >> 3) * 1024 + sw * 128;
+    uint8_t* prow = sP + (col0 >> 6) * kT16Sub + (row >> 3) * 1024 + sw * 128;
+    const int pch = (col0 >> 3) & 7;                              // first 16-byte chunk of this half
     for (int j = 0; j < n_kv && ok; ++j) {
       const int sb = j & 1, kv0 = kv_lo + j * kT16Kv;
       if (!wait_all(&s_full[sb], (j >> 1) & 1, 0x8d0)) { ok = false; break; }
       tc_fence_after();
-      const uint32_t ts = tS + sb * 128 + t_lane;
+      const uint32_t ts = tS + sb * kT16Kv + t_lane;
       const int vis = row_live ? pos + 1 - kv0 : 0, hid = lo_pos - kv0;       // visible columns [hid, vis)
-      uint32_t sr[2][32];
+      uint32_t sr[HC / 32][32];
 #pragma unroll
-      for (int c = 0; c < 2; ++c) tmem_ld_32x32b_x32(ts + col0 + c * 32, sr[c]);
+      for (int c = 0; c < HC / 32; ++c) tmem_ld_32x32b_x32(ts + col0 + c * 32, sr[c]);
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&s_free[sb]);
       if (capped) {
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
+        for (int c = 0; c < HC / 32; ++c)
 #pragma unroll
           for (int i = 0; i < 32; ++i) sr[c][i] = __float_as_uint(capped_score(__uint_as_float(sr[c][i]), p.cap_in, p.cap_out));
       }
       if (biased) {
         const float mul = capped ? 1.f : p.scale_log2;
         const int back = pos - kv0 - col0;                            // distance of this thread's first column
-        if (__all_sync(0xffffffffu, back - 63 >= p.reach)) {
+        if (__all_sync(0xffffffffu, back - (HC - 1) >= p.reach)) {
 #pragma unroll
-          for (int c = 0; c < 2; ++c)
+          for (int c = 0; c < HC / 32; ++c)
 #pragma unroll
             for (int i = 0; i < 32; ++i) sr[c][i] = __float_as_uint(fmaf(__uint_as_float(sr[c][i]), mul, bias_far));
         } else {
 #pragma unroll
-          for (int c = 0; c < 2; ++c)
+          for (int c = 0; c < HC / 32; ++c)
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
               const float bv = bias_row[min(max(back - c * 32 - i, 0), p.reach)] * bias_mul;
@@ -297,10 +303,10 @@ attn_prefill_tc16_kernel(const __grid_constant__ CUtensorMap tmap_q, const Tc16P
             }
         }
       }
-      const bool full = __all_sync(0xffffffffu, vis >= col0 + 64 && hid <= col0);
+      const bool full = __all_sync(0xffffffffu, vis >= col0 + HC && hid <= col0);
       if (!full) {
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
+        for (int c = 0; c < HC / 32; ++c)
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
             const int col = col0 + c * 32 + i;
@@ -309,7 +315,7 @@ attn_prefill_tc16_kernel(const __grid_constant__ CUtensorMap tmap_q, const Tc16P
       }
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int c = 0; c < 2; ++c)
+      for (int c = 0; c < HC / 32; ++c)
 #pragma unroll
         for (int i = 0; i < 32; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(sr[c][i]));
       const float mine = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
@@ -340,7 +346,7 @@ attn_prefill_tc16_kernel(const __grid_constant__ CUtensorMap tmap_q, const Tc16P
       float sum4[4] = {0.f, 0.f, 0.f, 0.f};
       const float mref = (m_new == -INFINITY) ? 0.f : m_new;      // rows that see nothing yet: every p is 0
 #pragma unroll
-      for (int c = 0; c < 2; ++c)
+      for (int c = 0; c < HC / 32; ++c)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           float e[8];
@@ -351,7 +357,7 @@ attn_prefill_tc16_kernel(const __grid_constant__ CUtensorMap tmap_q, const Tc16P
           }
           uint4 o;
           o.x = pack_bf16x2(e[0], e[1]); o.y = pack_bf16x2(e[2], e[3]); o.z = pack_bf16x2(e[4], e[5]); o.w = pack_bf16x2(e[6], e[7]);
-          *reinterpret_cast<uint4*>(prow + (((c * 4 + q) ^ sw) << 4)) = o;
+          *reinterpret_cast<uint4*>(prow + (((pch + c * 4 + q) ^ sw) << 4)) = o;
         }
       l = l * alpha + (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
       m = m_new;
@@ -398,7 +404,8 @@ attn_prefill_tc16_kernel(const __grid_constant__ CUtensorMap tmap_q, const Tc16P
 
 template <int D>
 static int launch_tc16(const CUtensorMap& tq, const Tc16Params& p, int num_tiles, cudaStream_t st) {
-  constexpr int kSmem = (D / 64) * kT16Sub + 2 * kT16Sub + 2 * (D / 64) * kT16Sub + 4 * D * 128 + 256 + 1024;
+  constexpr int KV = tc16_kv(D);
+  constexpr int kSmem = (D / 64) * kT16Sub + (KV / 64) * kT16Sub + 2 * (D / 64) * KV * 128 + 2 * (KV / 64) * D * 128 + 256 + 1024;
   Tc16Params pp = p;
   int bytes = kSmem;
   pp.bias_ld = 0;
@@ -425,7 +432,7 @@ extern "C" int atlas_attn_prefill_tc16(const void* q, long long ldq, void* out, 
                                        const float* distance, int reach, unsigned long long* status, void* stream) {
   if (num_tiles <= 0) return 0;
   if (distance && reach < 0) return -2;
-  if ((D != 64 && D != 128) || block_size != kT16Page || Hq % Hkv || Hq / Hkv > kT16Rows || !(scale > 0.f)) return 1;
+  if ((D != 64 && D != 128 && D != 256) || block_size != kT16Page || Hq % Hkv || Hq / Hkv > kT16Rows || !(scale > 0.f)) return 1;
   if ((reinterpret_cast<uintptr_t>(q) & 15) || (ldq % 8) || (ldo % 8) || (reinterpret_cast<uintptr_t>(out) & 15)) return 1;
   EncodeTiledFn enc = tc_encode_fn();
   if (!enc) return -10;
@@ -448,5 +455,5 @@ extern "C" int atlas_attn_prefill_tc16(const void* q, long long ldq, void* out, 
   p.distance = distance; p.reach = reach; p.bias_ld = 0;
   if (softcap > 0.f) cap_constants(scale, softcap, &p.cap_in, &p.cap_out);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  return D == 64 ? launch_tc16<64>(tq, p, num_tiles, st) : launch_tc16<128>(tq, p, num_tiles, st);
+  return D == 64 ? launch_tc16<64>(tq, p, num_tiles, st) : D == 128 ? launch_tc16<128>(tq, p, num_tiles, st) : launch_tc16<256>(tq, p, num_tiles, st);
 }

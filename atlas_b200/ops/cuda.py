@@ -830,7 +830,7 @@ def _paged_attention_kv16(q, out, k_cache, v_cache, batch, scale, window, d, sca
                                             bt.data_ptr(), bt.stride(0), batch.seq_lens.data_ptr(), batch.query_start_loc.data_ptr(),
                                             0, nd, float(scale), Hq, Hkv, D, bs, window, splits, _ptr(po), _ptr(pml), st, chunk,
                                             _ptr(sinks), softcap, *bias), "attn_decode_kv16")
-    if batch.num_seqs > nd and not fp4 and _TC_PREFILL and bs == 16 and D <= 128 and Hq // Hkv <= 128:
+    if batch.num_seqs > nd and not fp4 and _TC_PREFILL and bs == 16 and (D <= 128 or D == 256) and Hq // Hkv <= 128:
         # tcgen05 tiles of 128 // G query tokens; 1 = a shape the kernel does not take
         tdev, n_tiles, _ = _tc_tiles(q, batch, nd, 128 // (Hq // Hkv))
         if not getattr(L, "_tc16_bound", False):
@@ -906,7 +906,7 @@ _TC_PREFILL = os.environ.get("ATLAS_ATTN_TC", "1") not in ("0", "false")
 
 
 def _tc_prefill_ok(q, Hq, Hkv, D, bs, window, k_cache) -> bool:
-    return (_TC_PREFILL and D == 128 and bs == 16 and not window and Hq % Hkv == 0 and (Hq // Hkv) in (1, 2, 4, 8)
+    return (_TC_PREFILL and D in (128, 256) and bs == 16 and not window and Hq % Hkv == 0 and (Hq // Hkv) in (1, 2, 4, 8)
             and q.dtype == torch.bfloat16 and k_cache.dtype == torch.float8_e4m3fn)
 
 

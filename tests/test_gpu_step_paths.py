@@ -169,3 +169,22 @@ def test_chunked_mamba2_against_64_bits(K, lens, snaps):
         assert _rel(res[0][0][rows], want) < 2 ** -9
         for slot, ref64 in [(i, kept[n])] + [(s, kept[r]) for r, s in stops.items()]:
             assert _rel(res[0][1][slot], ref64) < max(1e-6, _rel(res[1][1][slot], ref64))
+
+
+# ----------------------------------------------------------------------------- chunk attention of 256-wide heads
+@pytest.mark.parametrize("kv", [torch.float8_e4m3fn, torch.bfloat16])
+@pytest.mark.parametrize("Hq,Hkv,qlens,ctxs", [(16, 2, [300, 1, 37, 63], [0, 90, 1000, 77]), (8, 2, [64, 65, 129], [64, 63, 0]), (4, 4, [130, 16], [1, 500]),
+                                               (16, 1, [40], [200])])
+def test_chunk_attention_of_wide_heads(K, kv, Hq, Hkv, qlens, ctxs, monkeypatch):
+    """Head dim 256 on the tcgen05 path (64-token KV tiles): edges of query and KV tiles, contexts, several group sizes (16 heads a group is
+    taken with a bf16 cache only), beside the general kernel; the bounds are those of the 128-wide heads."""
+    from test_gpu_kernels import _attention_case
+    args = dict(qlens=qlens, ctxs=ctxs, kv_dtype=kv)
+    out, want = _attention_case(K, 256, Hq, Hkv, **args)
+    assert K.check_status() == 0
+    assert _rel(out, want) < 2e-2
+    torch.testing.assert_close(out.float(), want.float(), atol=3e-2, rtol=5e-2)
+    monkeypatch.setattr(K, "_TC_PREFILL", False)
+    old, _ = _attention_case(K, 256, Hq, Hkv, **args)
+    assert _rel(out, want) <= 1.05 * _rel(old, want)
+    assert _rel(out, old) < 2e-2
