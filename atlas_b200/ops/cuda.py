@@ -290,9 +290,9 @@ def gemm_plan(M: int, N: int, K: int, kind: int, sms: int) -> Tuple[int, int]:
     m_tiles = (M + 127) // 128
     if _FORCE_BLOCK_N:
         bn = _FORCE_BLOCK_N
-    elif kind == 0 and m_tiles * ((N + 255) // 256) >= 2 * sms and N % 256 == 0:
-        bn = 256          # bf16 accumulates in TMEM across K
-    elif kind == 1 and m_tiles * ((N + 255) // 256) >= sms and N % 256 == 0:
+    elif kind == 0 and m_tiles * ((N + 255) // 256) >= 2 * sms and -N % 256 * 16 <= N:
+        bn = 256          # bf16 accumulates in TMEM across K; a last tile that is cut off costs at most 1/16
+    elif kind == 1 and m_tiles * ((N + 255) // 256) >= sms and -N % 256 * 16 <= N:
         bn = 256          # fp8: half the per-k-group buffer handshakes per FLOP and 0.75x the shared-memory fill of 128
     elif m_tiles * ((N + 127) // 128) >= sms:
         bn = 128
