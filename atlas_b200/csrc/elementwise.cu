@@ -140,10 +140,13 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bf
 template <int ACT>
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const __nv_bfloat16* __restrict__ gu, long long ld, int I, __nv_bfloat16* y, long long ldy, uint8_t* q,
-                long long ldq, float* scale, long long scale_ld, const int* rows) {
+                long long ldq, float* scale, long long scale_ld, const int* rows, int n) {
   chain_trigger();
   chain_wait();
-  const int t = rows ? rows[blockIdx.x] : (int)blockIdx.x;      // rows on grid.x: row counts can exceed the 65535 limit of grid.y
+  // rows on grid.x: row counts can exceed the 65535 limit of grid.y; narrow rows share a block (blockDim.y whole warps of threads each)
+  const int item = (int)blockIdx.x * blockDim.y + threadIdx.y;
+  if (item >= n) return;
+  const int t = rows ? rows[item] : item;
   if (t < 0) return;
   const int e = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
   const bool live = e < I;
@@ -520,34 +523,73 @@ v_write_pages_kernel(const RopeKvParams p) {
   }
 }
 
-// y = rmsnorm(x) * w * silu(z), one warp per (token, head); x,z [T, H, D] with token strides
+// y = rmsnorm(x) * w * silu(z), one warp per kUnits (token, head) pairs; x, z [T, H, D] with token strides.  kPer: pairs of channels per
+// lane known at compile time (D = 64 kPer), all loads of a warp in flight together; 0: any even D.
+// Bound by memory: 8192 x 32 heads of 128 channels 106 us with a pair per warp, 72 us (2.8 TB/s).
+template <int kPer, int kUnits>
 __global__ void __launch_bounds__(128)
 gated_rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ z,
                      long long ldz, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* y, long long ldy, int T, int H,
                      int D, float eps) {
+  chain_trigger();
+  chain_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long unit = (long long)blockIdx.x * 4 + warp;
-  if (unit >= (long long)T * H) return;
-  const int t = (int)(unit / H), h = (int)(unit % H);
-  const __nv_bfloat16* xr = x + t * ldx + h * D;
-  const __nv_bfloat16* zr = z + t * ldz + h * D;
-  float ss = 0.f;
-  for (int e = lane * 2; e < D; e += 64) {
-    float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(xr + e));
-    ss += f.x * f.x + f.y * f.y;
-  }
-  ss = warp_sum(ss);
-  const float rstd = rsqrtf(ss / (float)D + eps);
-  for (int e = lane * 2; e < D; e += 64) {
-    float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(xr + e));
-    float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(zr + e));
-    float2 wv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(w + e));
+  const long long first = ((long long)blockIdx.x * 4 + warp) * kUnits, units = (long long)T * H;
+  auto scaled = [&](float2 f, float2 g, float2 wv, float rstd) {
     const float a = f.x * rstd * wv.x * (g.x / (1.f + __expf(-g.x)));
     const float b = f.y * rstd * wv.y * (g.y / (1.f + __expf(-g.y)));
-    *reinterpret_cast<__nv_bfloat162*>(y + t * ldy + h * D + e) = __floats2bfloat162_rn(a, b);
+    return __floats2bfloat162_rn(a, b);
+  };
+  if constexpr (kPer > 0) {
+    __nv_bfloat162 xv[kUnits][kPer], zv[kUnits][kPer], wv[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) wv[i] = *reinterpret_cast<const __nv_bfloat162*>(w + lane * 2 + 64 * i);
+#pragma unroll
+    for (int u = 0; u < kUnits; ++u) {
+      const long long unit = min(first + u, units - 1);
+      const long long t = unit / H, c = (unit % H) * D + lane * 2;
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        xv[u][i] = *reinterpret_cast<const __nv_bfloat162*>(x + t * ldx + c + 64 * i);
+        zv[u][i] = *reinterpret_cast<const __nv_bfloat162*>(z + t * ldz + c + 64 * i);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kUnits; ++u) {
+      float ss = 0.f;
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        const float2 f = __bfloat1622float2(xv[u][i]);
+        ss += f.x * f.x + f.y * f.y;
+      }
+      ss = warp_sum(ss);
+      const float rstd = rsqrtf(ss / (float)D + eps);
+      if (first + u < units) {
+        __nv_bfloat16* o = y + (first + u) / H * ldy + (first + u) % H * D + lane * 2;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i)
+          *reinterpret_cast<__nv_bfloat162*>(o + 64 * i) =
+              scaled(__bfloat1622float2(xv[u][i]), __bfloat1622float2(zv[u][i]), __bfloat1622float2(wv[i]), rstd);
+      }
+    }
+  } else {
+    if (first >= units) return;
+    const int t = (int)(first / H), h = (int)(first % H);
+    const __nv_bfloat16* xr = x + t * ldx + h * D;
+    const __nv_bfloat16* zr = z + t * ldz + h * D;
+    float ss = 0.f;
+    for (int e = lane * 2; e < D; e += 64) {
+      float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(xr + e));
+      ss += f.x * f.x + f.y * f.y;
+    }
+    ss = warp_sum(ss);
+    const float rstd = rsqrtf(ss / (float)D + eps);
+    for (int e = lane * 2; e < D; e += 64)
+      *reinterpret_cast<__nv_bfloat162*>(y + t * ldy + h * D + e) =
+          scaled(__bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(xr + e)), __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(zr + e)),
+                 __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(w + e)), rstd);
   }
 }
-
 
 // Per-row LoRA update ("batched gather matrix-vector"): y[t, col0 + n] += scaling_s * sum_r B_s[n, r] * (A_s[r, :] . x[t, :])
 // with s = slot[t] (0 = no adapter: the row is left alone).  One CTA per row: warps take the r dot products of the
@@ -594,6 +636,8 @@ lora_bgmv_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const long 
 // x[t, :] *= sigmoid(gate[t, :]) in place (the output gate of gated attention); n % 8 == 0
 __global__ void __launch_bounds__(256)
 sigmoid_gate_mul_kernel(__nv_bfloat16* x, long long ldx, const __nv_bfloat16* __restrict__ gate, long long ldg, int n) {
+  chain_trigger();
+  chain_wait();
   const long long t = blockIdx.x;
   for (int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8; c < n; c += gridDim.y * blockDim.x * 8) {
     float xv[8], gv[8];
@@ -609,6 +653,8 @@ sigmoid_gate_mul_kernel(__nv_bfloat16* x, long long ldx, const __nv_bfloat16* __
 __global__ void __launch_bounds__(256)
 shared_expert_blend_kernel(__nv_bfloat16* y, long long ldy, const __nv_bfloat16* __restrict__ s, long long lds,
                            const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ wg, int H) {
+  chain_trigger();
+  chain_wait();
   const long long t = blockIdx.x;
   __shared__ float red[8];
   float dot = 0.f;
@@ -696,10 +742,12 @@ extern "C" int atlas_silu_mul(const void* gu, long long ld, int T, int I, void* 
   if (T <= 0) return 0;
   if (I % 8 || (q && I % 128)) return -1;
   const int threads = min(256, (I / 8 + 31) / 32 * 32);      // whole warps: groups of 16 lanes share a scale
-  dim3 grid(T, (I / 8 + threads - 1) / threads);
-  launch_chain_if(T <= 256, silu_mul_kernel<0>, grid, dim3(threads), 0, reinterpret_cast<cudaStream_t>(stream),
+  // large steps of narrow rows (experts): several to a block (81920 rows of 512: 86 us with a row each, 46 us so)
+  const int per = T > 256 ? 256 / threads : 1;
+  dim3 grid((T + per - 1) / per, (I / 8 + threads - 1) / threads);
+  launch_chain_if(T <= 256, silu_mul_kernel<0>, grid, dim3(threads, per), 0, reinterpret_cast<cudaStream_t>(stream),
       reinterpret_cast<const __nv_bfloat16*>(gu), ld, I, reinterpret_cast<__nv_bfloat16*>(y), ldy,
-      reinterpret_cast<uint8_t*>(q), ldq, scale, scale_ld, rows);
+      reinterpret_cast<uint8_t*>(q), ldq, scale, scale_ld, rows, T);
   return cudaGetLastError() == cudaSuccess ? 0 : -20;
 }
 
@@ -710,7 +758,7 @@ extern "C" int atlas_gelu_tanh_mul(const void* gu, long long ld, int T, int I, v
   dim3 grid(T, (I / 8 + 255) / 256);
   launch_chain_if(T <= 256, silu_mul_kernel<1>, grid, dim3(256), 0, reinterpret_cast<cudaStream_t>(stream),
       reinterpret_cast<const __nv_bfloat16*>(gu), ld, I, reinterpret_cast<__nv_bfloat16*>(y), ldy,
-      reinterpret_cast<uint8_t*>(q), ldq, scale, scale_ld, static_cast<const int*>(nullptr));
+      reinterpret_cast<uint8_t*>(q), ldq, scale, scale_ld, static_cast<const int*>(nullptr), T);
   return cudaGetLastError() == cudaSuccess ? 0 : -20;
 }
 
@@ -780,9 +828,15 @@ extern "C" int atlas_gated_rmsnorm(const void* x, long long ldx, const void* z, 
   if (T <= 0) return 0;
   if (D % 2) return -1;
   const long long units = (long long)T * H;
-  gated_rmsnorm_kernel<<<(int)((units + 3) / 4), 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), ldx, reinterpret_cast<const __nv_bfloat16*>(z), ldz,
-      reinterpret_cast<const __nv_bfloat16*>(w), reinterpret_cast<__nv_bfloat16*>(y), ldy, T, H, D, eps);
+  auto run = [&](auto kern, int per_warp) {
+    launch_chain_if(T <= 256, kern, dim3((unsigned)((units + 4 * per_warp - 1) / (4 * per_warp))), dim3(128), 0, reinterpret_cast<cudaStream_t>(stream),
+                    reinterpret_cast<const __nv_bfloat16*>(x), ldx, reinterpret_cast<const __nv_bfloat16*>(z), ldz,
+                    reinterpret_cast<const __nv_bfloat16*>(w), reinterpret_cast<__nv_bfloat16*>(y), ldy, T, H, D, eps);
+  };
+  // four pairs a warp where that leaves every SM several blocks
+  if (D != 128) run(gated_rmsnorm_kernel<0, 1>, 1);
+  else if (units >= 16384) run(gated_rmsnorm_kernel<2, 4>, 4);
+  else run(gated_rmsnorm_kernel<2, 1>, 1);
   return cudaGetLastError() == cudaSuccess ? 0 : -20;
 }
 
@@ -810,7 +864,7 @@ extern "C" int atlas_sigmoid_gate_mul(void* x, long long ldx, const void* gate, 
   if (T <= 0 || n <= 0) return 0;
   if (n % 8 || ldx % 8 || ldg % 8 || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(gate) & 15)) return -1;
   dim3 grid(T, (n / 8 + 255) / 256);
-  sigmoid_gate_mul_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  launch_chain_if(T <= 256, sigmoid_gate_mul_kernel, grid, dim3(256), 0, reinterpret_cast<cudaStream_t>(stream),
       reinterpret_cast<__nv_bfloat16*>(x), ldx, reinterpret_cast<const __nv_bfloat16*>(gate), ldg, n);
   return cudaGetLastError() == cudaSuccess ? 0 : -20;
 }
@@ -819,7 +873,7 @@ extern "C" int atlas_shared_expert_blend(void* y, long long ldy, const void* s, 
                                          const void* wg, int T, int H, void* stream) {
   if (T <= 0) return 0;
   if (H % 8 || ldy % 8 || lds % 8 || ldx % 8) return -1;
-  shared_expert_blend_kernel<<<T, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  launch_chain_if(T <= 256, shared_expert_blend_kernel, dim3(T), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream),
       reinterpret_cast<__nv_bfloat16*>(y), ldy, reinterpret_cast<const __nv_bfloat16*>(s), lds,
       reinterpret_cast<const __nv_bfloat16*>(x), ldx, reinterpret_cast<const __nv_bfloat16*>(wg), H);
   return cudaGetLastError() == cudaSuccess ? 0 : -20;

@@ -29,6 +29,8 @@ struct GdnParams {
 template <int DK>
 __global__ void __launch_bounds__(256)
 gdn_recurrent_kernel(const GdnParams p) {
+  chain_trigger();
+  chain_wait();
   const int hv = blockIdx.x, bseq = blockIdx.y;
   const int j = threadIdx.x;                   // column of the state (value dim)
   const int DV = p.Dv;
@@ -338,9 +340,9 @@ extern "C" int atlas_gdn_recurrent(const void* y, long long ldy, const void* a, 
   dim3 grid(Hv, B);
   int threads = ((max(Dv, max(Dk, 65)) + 31) / 32) * 32;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (Dk == 128) gdn_recurrent_kernel<128><<<grid, threads, 0, st>>>(p);
-  else if (Dk == 64) gdn_recurrent_kernel<64><<<grid, threads, 0, st>>>(p);
-  else if (Dk == 32) gdn_recurrent_kernel<32><<<grid, threads, 0, st>>>(p);
+  if (Dk == 128) launch_chain(gdn_recurrent_kernel<128>, grid, dim3(threads), 0, st, p);
+  else if (Dk == 64) launch_chain(gdn_recurrent_kernel<64>, grid, dim3(threads), 0, st, p);
+  else if (Dk == 32) launch_chain(gdn_recurrent_kernel<32>, grid, dim3(threads), 0, st, p);
   else return -2;
   return cudaGetLastError() == cudaSuccess ? 0 : -20;
 }

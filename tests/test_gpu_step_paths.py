@@ -71,10 +71,12 @@ def test_expert_products_touch_live_rows_only(K, T, E, hot):
     assert _rel(got, want) < 0.02 if float(want.abs().max()) > 0 else float(got.abs().max()) == 0
 
 
-def test_expert_row_lists(K):
-    """align: every routed pair has a row of its own inside its expert's segment, and the tiles say how many rows live."""
+@pytest.mark.parametrize("T,k", [(75, 4), (1023, 4), (1024, 4), (2731, 3)])
+def test_expert_row_lists(K, T, k):
+    """align: every routed pair has a row of its own inside its expert's segment, and the tiles say how many rows live (one CTA; a
+    cluster from 4096 pairs on, with a remainder behind the last four ids)."""
     torch.manual_seed(0)
-    T, k, E, lo, n = 75, 4, 32, 8, 16
+    E, lo, n = 32, 8, 16
     ids = torch.stack([torch.randperm(E)[:k] for _ in range(T)]).int().to(DEV)
     tiles = T * k // 128 + min(T * k, n)
     slot, rows = torch.empty(T * k, dtype=torch.int32, device=DEV), torch.full((tiles * 128,), -7, dtype=torch.int32, device=DEV)
@@ -83,15 +85,58 @@ def test_expert_row_lists(K):
                                      tiles * 128, K._status_ptr[K._dev(ids)], K._stream()), "moe_align")
     live = int(nt)
     assert int(tr[:live].sum()) == int(((ids >= lo) & (ids < lo + n)).sum())
-    flat, slot = ids.flatten().tolist(), slot.tolist()
+    flat, slot, te, tr, rows = ids.flatten().tolist(), slot.tolist(), te.tolist(), tr.tolist(), rows.tolist()
     used = [s for s in slot if s >= 0]
     assert len(set(used)) == len(used)
     for i, (e, s) in enumerate(zip(flat, slot)):
         assert (s >= 0) == (lo <= e < lo + n)
         if s >= 0:
-            assert int(te[s // 128]) == e - lo and s % 128 < int(tr[s // 128]) and int(rows[s]) == i // k
+            assert te[s // 128] == e - lo and s % 128 < tr[s // 128] and rows[s] == i // k
     for t in range(live):
-        assert (rows[t * 128 + int(tr[t]):(t + 1) * 128] == -1).all()
+        assert all(r == -1 for r in rows[t * 128 + tr[t]:(t + 1) * 128])
+
+
+@pytest.mark.parametrize("E,k,dtype", [(33, 5, torch.bfloat16), (64, 8, torch.float32), (256, 8, torch.bfloat16), (257, 32, torch.bfloat16),
+                                       (512, 10, torch.bfloat16), (513, 10, torch.float32), (1024, 4, torch.bfloat16)])
+def test_route_picks_the_largest(K, E, k, dtype):
+    """Largest logits first, the lowest expert among equal ones (coarse logits, so that many are), minus infinity last; weights sum to 1."""
+    torch.manual_seed(E)
+    logits = (torch.randn(19, E, device=DEV) * 4).round().div(2).to(dtype)
+    logits[3] = -1.5
+    logits[4, k:] = -float("inf")
+    w, ids = K.moe_route(logits, k, True, "softmax")
+    order = torch.sort(logits.double(), dim=-1, descending=True, stable=True)
+    assert torch.equal(ids.long(), order.indices[:, :k])
+    want = order.values[:, :k].softmax(-1)
+    assert float((w.double() - want).abs().max()) < 1e-5
+
+
+@pytest.mark.parametrize("T,H,D", [(1, 3, 128), (7, 5, 128), (600, 31, 128), (513, 32, 128), (5, 3, 96)])
+def test_gated_norm_of_heads(K, T, H, D):
+    torch.manual_seed(T)
+    x, z, w = (torch.randn(*s, device=DEV).bfloat16() for s in ((T, H, D), (T, H, D), (D,)))
+    y = K.gated_rmsnorm(x, z, w, 1e-6).double()
+    xd = x.double()
+    want = xd * torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-6) * w.double() * torch.nn.functional.silu(z.double())
+    assert float(((y - want).abs() / (want.abs() + 1e-3)).max()) < 2 ** -8
+
+
+@pytest.mark.parametrize("T,I", [(3, 512), (259, 128), (300, 512), (257, 2304), (1000, 384)])
+def test_silu_rows_share_blocks(K, T, I):
+    """Rows by index with gaps, several to a block: each is what it is alone, others stay."""
+    torch.manual_seed(T)
+    gu = torch.randn(T, 2 * I, device=DEV).bfloat16()
+    rows = torch.randperm(T)[:T - 1].int().to(DEV)
+    rows[::5] = -1
+    q, s = torch.zeros(T, I, dtype=torch.uint8, device=DEV), torch.zeros(I // 128, T, device=DEV)
+    K._check(K.lib().atlas_silu_mul(gu.data_ptr(), 2 * I, rows.numel(), I, None, 0, q.data_ptr(), I, s.data_ptr(), T, rows.data_ptr(), K._stream()), "silu_mul")
+    one, sc = K.silu_mul(gu[:200].contiguous(), quant=True)
+    got = torch.zeros(T, dtype=torch.bool, device=DEV)
+    got[rows[rows >= 0].long()] = True
+    m = min(200, T)
+    live = got[:m]
+    assert torch.equal(q[:m][live], one[:m].view(torch.uint8)[live]) and torch.equal(s[:, :m].t()[live], sc[:m][live])
+    assert int(q[~got].sum()) == 0 and float(s.t()[~got].abs().sum()) == 0
 
 
 # ----------------------------------------------------------------------------- decode graphs of Gated DeltaNet models
