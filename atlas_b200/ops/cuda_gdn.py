@@ -11,7 +11,8 @@ from . import cuda as K
 _vp, _ll, _i = C.c_void_p, C.c_longlong, C.c_int
 _bound = False
 USE_CHUNKED = True          # tests switch this off to compare the two kernels
-CHUNK_MIN_ROWS = 32
+CHUNK_MIN_ROWS = 32         # rows of the longest sequence from which a step takes the chunked kernels
+CHUNK_ROWS_OF_SEQ = 16      # they leave sequences with fewer rows (decode rows beside a prompt) to the recurrence
 
 
 def _lib():
@@ -19,9 +20,11 @@ def _lib():
     lib = K.lib()
     if not _bound:
         lib.atlas_gdn_recurrent.argtypes = [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp,
-                                            _vp, _i, _i, _i, _i, _i, _i, _i, _vp]
+                                            _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp]
         lib.atlas_gdn_chunked.argtypes = [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _i,
-                                          _i, _i, _i, _i, _i, _i, _vp]
+                                          _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp]
+        lib.atlas_gdn_chunked_bytes.argtypes = [_i, _i, _i, _i, _i, C.POINTER(_i)]
+        lib.atlas_gdn_chunked_bytes.restype = _ll
         _bound = True
     return lib
 
@@ -86,19 +89,21 @@ def _run(layer, mixed, a, b, meta: _Meta, state, commit: bool):
     cuda_recurrent.conv_silu(mixed, cw, None, conv, meta, y, commit, silu=2)
     rc = 1
     if USE_CHUNKED and meta.chunk_ok and commit and layer.dk == 128 and layer.dv == 128:
+        work = torch.empty(lib.atlas_gdn_chunked_bytes(T, meta.B, meta.snaps, layer.hk, layer.hv, C.byref(_i())), dtype=torch.uint8, device=mixed.device)
         rc = lib.atlas_gdn_chunked(y.data_ptr(), Cc, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0),
                                    layer.A_log.data_ptr(), layer.dt_bias.data_ptr(), h.data_ptr(), out.data_ptr(),
                                    layer.hv * layer.dv, meta.qsl.data_ptr(), meta.slots.data_ptr(), meta.has.data_ptr(),
-                                   meta.snap_rows.data_ptr(), meta.snap_slots.data_ptr(), meta.snaps, meta.B, layer.hk,
-                                   layer.hv, layer.dk, layer.dv, 1, st)
+                                   meta.snap_rows.data_ptr(), meta.snap_slots.data_ptr(), meta.snaps, T, meta.B, layer.hk,
+                                   layer.hv, layer.dk, layer.dv, 1, CHUNK_ROWS_OF_SEQ, work.data_ptr(), st)
         if rc != 1:
             K._check(rc, "gdn_chunked")
-    if rc == 1:
-      K._check(lib.atlas_gdn_recurrent(y.data_ptr(), Cc, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0),
-                                       layer.A_log.data_ptr(), layer.dt_bias.data_ptr(), h.data_ptr(), out.data_ptr(),
-                                       layer.hv * layer.dv, meta.qsl.data_ptr(), meta.slots.data_ptr(), meta.has.data_ptr(),
-                                       K._ptr(meta.limit), meta.snap_rows.data_ptr(), meta.snap_slots.data_ptr(), meta.snaps,
-                                       meta.B, layer.hk, layer.hv, layer.dk, layer.dv, 1 if commit else 0, st), "gdn_recurrent")
+    if rc == 1 or meta.shortest < CHUNK_ROWS_OF_SEQ:           # the latter: sequences that the chunked kernels have left out
+        K._check(lib.atlas_gdn_recurrent(y.data_ptr(), Cc, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0),
+                                         layer.A_log.data_ptr(), layer.dt_bias.data_ptr(), h.data_ptr(), out.data_ptr(),
+                                         layer.hv * layer.dv, meta.qsl.data_ptr(), meta.slots.data_ptr(), meta.has.data_ptr(),
+                                         K._ptr(meta.limit), meta.snap_rows.data_ptr(), meta.snap_slots.data_ptr(), meta.snaps,
+                                         meta.B, layer.hk, layer.hv, layer.dk, layer.dv, 1 if commit else 0,
+                                         0 if rc == 1 else CHUNK_ROWS_OF_SEQ, st), "gdn_recurrent")
     cuda_recurrent.conv_advance(mixed, layer.W, conv, meta, commit)
     return out
 

@@ -167,6 +167,92 @@ def test_delta_net_decode_graph_equals_eager_steps(K, n):
     assert all(torch.equal(a, b) for a, b in zip(*outs))
 
 
+# ----------------------------------------------------------------------------- chunked delta rule
+def _delta_rule(y, a, b, a_log, dt_bias, h, hk, hv, stops):
+    """The recurrence in 64 bits: outputs, and the state after every row count in ``stops``."""
+    y, a, b, h = y.double(), a.double(), b.double(), h.double().clone()
+    n, d, out, kept = y.shape[0], 128, [], {}
+    unit = lambda t: t * torch.rsqrt(t.square().sum(-1, keepdim=True) + 1e-6)
+    q, k = unit(y[:, :hk * d].view(n, hk, d)) / d ** 0.5, unit(y[:, hk * d:2 * hk * d].view(n, hk, d))
+    q, k, v = q.repeat_interleave(hv // hk, 1), k.repeat_interleave(hv // hk, 1), y[:, 2 * hk * d:].view(n, hv, d)
+    decay = torch.exp(-torch.exp(a_log.double()) * torch.nn.functional.softplus(a + dt_bias.double()))
+    beta = torch.sigmoid(b)
+    for t in range(n):
+        h = h * decay[t][:, None, None]
+        h = h + k[t][:, :, None] * ((v[t] - torch.einsum("hkv,hk->hv", h, k[t])) * beta[t][:, None])[:, None]
+        out.append(torch.einsum("hkv,hk->hv", h, q[t]).flatten())
+        if t + 1 in stops:
+            kept[t + 1] = h.clone()
+    return torch.stack(out), kept
+
+
+@pytest.mark.parametrize("lens,snaps,like", [([1], {}, 0.0), ([64, 63, 65], {}, 0.0), ([300, 1, 128], {0: [(1, 6), (64, 7), (200, 8)], 2: [(128, 9)]}, 0.0),
+                                             ([515], {0: [(130, 3)]}, 0.95)])
+def test_chunked_delta_rule_against_64_bits(K, lens, snaps, like):
+    """Edges of the 64-row chunks, snapshot rows inside and on them, and keys that are nearly the same (``like``: the inverse inside a
+    chunk is then far from the identity).  Every product rounds its operands to TF32 (2^-12 in the norm), of which a state and an
+    output take about ten in a chain: 2.5e-3; outputs are rounded to bf16 besides (2^-9 at most)."""
+    import ctypes
+    from atlas_b200.ops import cuda_gdn
+    torch.manual_seed(sum(lens))
+    hk, hv, d, T, B = 2, 4, 128, sum(lens), len(lens)
+    y = torch.randn(T, (2 * hk + hv) * d, device=DEV)
+    base = torch.randn(1, hk * d, device=DEV)
+    y[:, hk * d:2 * hk * d] = like * base + (1 - like * like) ** 0.5 * y[:, hk * d:2 * hk * d]
+    y = y.bfloat16()
+    a, b = torch.randn(T, hv, device=DEV).bfloat16(), torch.randn(T, hv, device=DEV).bfloat16()
+    a_log, dt_bias = torch.linspace(-3, 2, hv, device=DEV), torch.linspace(-4, 1, hv, device=DEV)
+    h0 = torch.randn(12, hv, d, d, device=DEV) * 0.1
+    has = [i % 2 == 0 for i in range(B)]
+    meta = cuda_gdn._Meta(lens, list(range(B)), has, DEV, snaps)
+    h, out, lib = h0.clone(), torch.empty(T, hv * d, dtype=torch.bfloat16, device=DEV), cuda_gdn._lib()
+    heads = ctypes.c_int()
+    work = torch.empty(lib.atlas_gdn_chunked_bytes(T, B, meta.snaps, hk, hv, ctypes.byref(heads)), dtype=torch.uint8, device=DEV)
+    assert heads.value == hv
+    K._check(lib.atlas_gdn_chunked(y.data_ptr(), y.stride(0), a.data_ptr(), hv, b.data_ptr(), hv, a_log.data_ptr(), dt_bias.data_ptr(), h.data_ptr(),
+                                   out.data_ptr(), hv * d, meta.qsl.data_ptr(), meta.slots.data_ptr(), meta.has.data_ptr(), meta.snap_rows.data_ptr(),
+                                   meta.snap_slots.data_ptr(), meta.snaps, T, B, hk, hv, d, d, 1, 1, work.data_ptr(), K._stream()), "gdn_chunked")
+    t = 0
+    for i, n in enumerate(lens):
+        rows = slice(t, t + n)
+        t += n
+        stops = {r: s for r, s in snaps.get(i, [])}
+        want, kept = _delta_rule(y[rows], a[rows], b[rows], a_log, dt_bias, h0[i] * has[i], hk, hv, set(stops) | {n})
+        assert _rel(out[rows], want) < 2.5e-3 + 2 ** -9
+        assert _rel(h[i], kept[n]) < 2.5e-3
+        for r, s in stops.items():
+            assert _rel(h[s], kept[r]) < 2.5e-3
+
+
+def test_chunked_delta_rule_workspace_is_bounded(K):
+    """Long steps go through the heads in groups, with the results of one group."""
+    import ctypes
+    from atlas_b200.ops import cuda_gdn
+    lib, heads = cuda_gdn._lib(), ctypes.c_int()
+    small = lib.atlas_gdn_chunked_bytes(8192, 1, 0, 16, 32, ctypes.byref(heads))
+    assert heads.value == 32 and small <= 256 << 20
+    assert lib.atlas_gdn_chunked_bytes(40000, 3, 2, 16, 32, ctypes.byref(heads)) <= 256 << 20 and heads.value == 8
+    torch.manual_seed(1)
+    hk, hv, d, T = 3, 3, 128, 150000
+    assert lib.atlas_gdn_chunked_bytes(T, 1, 0, hk, hv, ctypes.byref(heads)) <= 256 << 20 and heads.value == 1
+    y = torch.randn(T, (2 * hk + hv) * d, device=DEV).bfloat16()
+    a, b = torch.randn(T, hv, device=DEV).bfloat16(), torch.randn(T, hv, device=DEV).bfloat16()
+    a_log, dt_bias = torch.zeros(hv, device=DEV), torch.zeros(hv, device=DEV)
+    res = []
+    for only in (None, 2):                    # all heads; the last one alone, as a model of one head
+        n = hv if only is None else 1
+        yy = y if only is None else torch.cat([y[:, (only + i) * d:(only + i + 1) * d] for i in (0, hk, 2 * hk)], 1).contiguous()
+        aa, bb = (a, b) if only is None else (a[:, only:only + 1].contiguous(), b[:, only:only + 1].contiguous())
+        meta = cuda_gdn._Meta([T], [0], [False], DEV)
+        h, out = torch.zeros(1, n, d, d, device=DEV), torch.empty(T, n * d, dtype=torch.bfloat16, device=DEV)
+        work = torch.empty(lib.atlas_gdn_chunked_bytes(T, 1, 0, n, n, ctypes.byref(heads)), dtype=torch.uint8, device=DEV)
+        K._check(lib.atlas_gdn_chunked(yy.data_ptr(), yy.stride(0), aa.data_ptr(), n, bb.data_ptr(), n, a_log.data_ptr(), dt_bias.data_ptr(),
+                                       h.data_ptr(), out.data_ptr(), n * d, meta.qsl.data_ptr(), meta.slots.data_ptr(), meta.has.data_ptr(),
+                                       meta.snap_rows.data_ptr(), meta.snap_slots.data_ptr(), 0, T, 1, n, n, d, d, 1, 1, work.data_ptr(), K._stream()), "gdn_chunked")
+        res.append((out.view(T, n, d)[:, -1].clone(), h[0, -1].clone()))
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+
+
 # ----------------------------------------------------------------------------- chunked Mamba-2
 def _mamba_scan(u, dt, a_log, skip, bias, h, H, G, stops):
     """The recurrence in 64 bits over rows [x | B | C]: outputs, and the state after every row count in ``stops``."""
