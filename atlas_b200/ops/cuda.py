@@ -296,8 +296,14 @@ def gemm_plan(M: int, N: int, K: int, kind: int, sms: int) -> Tuple[int, int]:
         bn = 256          # fp8: half the per-k-group buffer handshakes per FLOP and 0.75x the shared-memory fill of 128
     elif m_tiles * ((N + 127) // 128) >= sms:
         bn = 128
-    elif kind == 1 and m_tiles == 1 and K >= 8192 and N % 128 == 0:
-        bn = 128          # decode rows, long K: fewer, wider tiles and more K splits (128 x 4096 x 14336: 35.5 -> 31.1 us)
+    elif m_tiles == 1 and K >= 8192 and N % 128 == 0:
+        # decode rows, long K: fewer, wider tiles and more K splits (FP8 128 x 4096 x 14336: 35.5 -> 31.1 us; bf16 32 x 4096 x 21504:
+        # 56.3 -> 38.2 us, x 8192: 25.6 -> 19.8 us)
+        bn = 128
+    elif m_tiles == 1 and (N + 63) // 64 > sms:
+        # decode rows: one wave of 128-wide tiles (up to sms: the rule above) where 64-wide ones would leave a second wave nearly empty
+        # (bf16 18560 x 4096: 43.8 -> 32.2 us, 12672 x 2048: 22.8 -> 15.3; FP8 12352 x 2048: 16.2 -> 11.5; 9216 x 2048, 144 tiles: 9.9, 11.0)
+        bn = 128
     else:
         bn = 64 if N >= 64 * 8 else 64
     tiles = m_tiles * ((N + bn - 1) // bn)
