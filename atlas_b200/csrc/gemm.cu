@@ -188,6 +188,10 @@ ATLAS_DEVICE ItemPos item_pos(const GemmParams& p, int item, int m_tiles) {
   ItemPos r;
   if (p.cluster_splits > 1) {
     r.m_tile = 0; r.n_tile = item / p.cluster_splits; r.split = item % p.cluster_splits;
+  } else if (p.tile_expert != nullptr) {
+    // Experts: the column tiles of a row tile one after the other, so that its rows come from HBM once and from L2 after that (row tiles
+    // first read 230 MB of rows again for every column tile: 8192 tokens x 10 of 512 experts, 878 and 844 us a layer).
+    r.m_tile = item / p.n_tiles; r.n_tile = item % p.n_tiles; r.split = 0;
   } else {
     r.m_tile = item % m_tiles;
     const int rest = item / m_tiles;
