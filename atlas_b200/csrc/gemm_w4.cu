@@ -30,16 +30,22 @@ constexpr int kW4EpiWarps = 4;
 constexpr int kW4Threads = 32 * (2 + kW4ConvWarps + kW4EpiWarps + 1);
 constexpr int kW4AWarp = 2 + kW4ConvWarps + kW4EpiWarps;      // index of the A-tile producer warp
 
-template <int BLOCK_N>
+// ROWS 256: two row tiles share every converted slice.  What bounds a slice of one tile is its conversion (ALU work of eight warps, three to
+// four times the MMAs): 8192 x 4096 x 4096 445 us with one tile, 292 us with two; 36016 routed rows on 128 experts of 1536 x 2048 and
+// 2048 x 768 741 and 652 us for the pair of products.
+template <int BLOCK_N, int ROWS>
 struct W4Cfg {
-  static constexpr int kABytes = kW4BlockM * 128;       // 128 rows x 64 bf16
+  static constexpr int kTiles = ROWS / kW4BlockM;
+  static constexpr int kATile = kW4BlockM * 128;        // 128 rows x 64 bf16
+  static constexpr int kABytes = kTiles * kATile;
   static constexpr int kBBytes = BLOCK_N * 128;         // converted operand, same layout as a TMA-swizzled tile
   static constexpr int kPBytes = BLOCK_N * 32;          // packed nibbles of one 64-wide K slice
   static constexpr int kStageBytes = kABytes + kBBytes;   // operand stage: A + converted B
-  static constexpr int kStages = BLOCK_N == 128 ? 4 : 5;
+  static constexpr int kStages = kTiles == 2 ? 3 : (BLOCK_N == 128 ? 4 : 5);
   static constexpr int kPStages = 16;                     // packed-slice ring (the HBM stream)
   static constexpr int kAccStages = 2;
-  static constexpr int kTmemCols = kAccStages * BLOCK_N;
+  static constexpr int kAccCols = kTiles * BLOCK_N;
+  static constexpr int kTmemCols = kAccStages * kAccCols;
   static constexpr int kGsBytes = 2 * BLOCK_N * 4;      // global scales of the tile's columns, double buffered
   static constexpr int kOperandBytes = kStages * kStageBytes;
   static constexpr int kSmemBytes = kOperandBytes + kPStages * kPBytes + kGsBytes + 1024 /*align*/ + 512 /*barriers*/;
@@ -56,6 +62,7 @@ struct W4Params {
   int b_rows;                 // rows of B (N, or E * N for the grouped form)
   int vec_ok;
   const int* tile_expert;     // nullptr = plain GEMM
+  const int* unit_tile;       // first tiles of pairs of one expert's tiles, num_m_tiles_ptr[1] of them
   const int* num_m_tiles_ptr;
   int expert_n;
 };
@@ -80,11 +87,27 @@ ATLAS_DEVICE __half2 e4m3_to_half2(uint32_t byte) {
   return __half2half2(*reinterpret_cast<__half*>(&h));
 }
 
-template <int BLOCK_N>
+// What a CTA works on next: `count` row tiles from t0 on (of one expert) times one column tile.
+struct W4Work { int t0, count, n_tile; };
+template <int TILES, typename F>
+ATLAS_DEVICE bool w4_unit(const W4Params& p, int item, int m_tiles, F work) {
+  // Experts: the column tiles of a unit one after the other, so that its rows come from HBM once and from L2 after that (row tiles
+  // first read 190 MB of rows again for every column tile: the pair of products 652, so 567 us).
+  if (p.tile_expert) {
+    const int u = item / p.n_tiles, t0 = TILES == 1 ? u : p.unit_tile[u];
+    const bool two = TILES == 2 && t0 + 1 < m_tiles && p.tile_expert[t0] == p.tile_expert[t0 + 1];
+    return work(W4Work{t0, two ? 2 : 1, item % p.n_tiles});
+  }
+  const int units = (m_tiles + TILES - 1) / TILES, t0 = item % units * TILES;
+  return work(W4Work{t0, min(TILES, m_tiles - t0), item / units});
+}
+
+template <int BLOCK_N, int ROWS>
 __global__ void __launch_bounds__(kW4Threads, 1)
 gemm_w4a16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_p,
                           const W4Params p) {
-  using Cfg = W4Cfg<BLOCK_N>;
+  using Cfg = W4Cfg<BLOCK_N, ROWS>;
+  constexpr int kTiles = Cfg::kTiles;
   constexpr int kStages = Cfg::kStages;
   constexpr int kAcc = Cfg::kAccStages;
   constexpr uint32_t kIdesc = make_idesc(kW4BlockM, BLOCK_N, 1u);      // bf16 x bf16
@@ -139,7 +162,7 @@ gemm_w4a16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   const uint32_t tmem_base = *tmem_slot;
 
   const int m_tiles = p.tile_expert ? *p.num_m_tiles_ptr : p.m_tiles;
-  const int total_items = m_tiles * p.n_tiles;
+  const int total_items = (kTiles == 2 && p.tile_expert ? p.num_m_tiles_ptr[1] : (m_tiles + kTiles - 1) / kTiles) * p.n_tiles;
   const int M_rows = p.tile_expert ? m_tiles * kW4BlockM : p.M;
 
   if (warp == 0) {
@@ -148,14 +171,16 @@ gemm_w4a16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       uint32_t ps = 0, pphase = 0;
       bool ok = true;
       for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-        const int m_tile = item % m_tiles, n_tile = item / m_tiles;
-        const int brow0 = (p.tile_expert ? p.tile_expert[m_tile] * p.expert_n : 0) + n_tile * BLOCK_N;
-        for (int kb = 0; kb < p.k_blocks; ++kb) {
-          if (!mbar_wait(&p_empty[ps], pphase ^ 1u, abort_flag, p.status, 0x700)) { ok = false; break; }
-          mbar_expect_tx(&p_full[ps], Cfg::kPBytes);
-          tma_load_2d(pring + ps * Cfg::kPBytes, &tmap_p, &p_full[ps], kb * 32, brow0);
-          if (++ps == kPStages) { ps = 0; pphase ^= 1u; }
-        }
+        ok = w4_unit<kTiles>(p, item, m_tiles, [&](const W4Work wk) {
+          const int brow0 = (p.tile_expert ? p.tile_expert[wk.t0] * p.expert_n : 0) + wk.n_tile * BLOCK_N;
+          for (int kb = 0; kb < p.k_blocks; ++kb) {
+            if (!mbar_wait(&p_empty[ps], pphase ^ 1u, abort_flag, p.status, 0x700)) return false;
+            mbar_expect_tx(&p_full[ps], Cfg::kPBytes);
+            tma_load_2d(pring + ps * Cfg::kPBytes, &tmap_p, &p_full[ps], kb * 32, brow0);
+            if (++ps == kPStages) { ps = 0; pphase ^= 1u; }
+          }
+          return true;
+        });
       }
       if (!ok)
         for (int i = 0; i < 64; ++i) __nanosleep(1000);       // let copies in flight land before shared memory goes away
@@ -166,13 +191,16 @@ gemm_w4a16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       uint32_t stage = 0, phase = 0;
       bool ok = true;
       for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-        const int m_tile = item % m_tiles;
-        for (int kb = 0; kb < p.k_blocks; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, 0x701)) { ok = false; break; }
-          mbar_expect_tx(&full[stage], Cfg::kABytes);
-          tma_load_2d(smem + stage * Cfg::kStageBytes, &tmap_a, &full[stage], kb * 64, m_tile * kW4BlockM);
-          if (++stage == kStages) { stage = 0; phase ^= 1u; }
-        }
+        ok = w4_unit<kTiles>(p, item, m_tiles, [&](const W4Work wk) {
+          for (int kb = 0; kb < p.k_blocks; ++kb) {
+            if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, 0x701)) return false;
+            mbar_expect_tx(&full[stage], wk.count * Cfg::kATile);
+            for (int i = 0; i < wk.count; ++i)
+              tma_load_2d(smem + stage * Cfg::kStageBytes + i * Cfg::kATile, &tmap_a, &full[stage], kb * 64, (wk.t0 + i) * kW4BlockM);
+            if (++stage == kStages) { stage = 0; phase ^= 1u; }
+          }
+          return true;
+        });
       }
       if (!ok)
         for (int i = 0; i < 64; ++i) __nanosleep(1000);
@@ -183,25 +211,29 @@ gemm_w4a16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       uint32_t stage = 0, phase = 0, acc_iter = 0;
       bool ok = true;
       for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-        const uint32_t buf = acc_iter % kAcc, aph = (acc_iter / kAcc) & 1u;
-        if (!mbar_wait(&acc_empty[buf], aph ^ 1u, abort_flag, p.status, 0x710)) break;
-        tc_fence_after();
-        for (int kb = 0; kb < p.k_blocks; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag, p.status, 0x711)) { ok = false; break; }
-          if (!mbar_wait(&conv[stage], phase, abort_flag, p.status, 0x712)) { ok = false; break; }
+        ok = w4_unit<kTiles>(p, item, m_tiles, [&](const W4Work wk) {
+          const uint32_t buf = acc_iter % kAcc, aph = (acc_iter / kAcc) & 1u;
+          if (!mbar_wait(&acc_empty[buf], aph ^ 1u, abort_flag, p.status, 0x710)) return false;
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
-          const uint64_t adesc = make_smem_desc_sw128(sa);
-          const uint64_t bdesc = make_smem_desc_sw128(sa + Cfg::kABytes);
-          const uint32_t d = tmem_base + buf * BLOCK_N;
+          for (int kb = 0; kb < p.k_blocks; ++kb) {
+            if (!mbar_wait(&full[stage], phase, abort_flag, p.status, 0x711)) return false;
+            if (!mbar_wait(&conv[stage], phase, abort_flag, p.status, 0x712)) return false;
+            tc_fence_after();
+            const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
+            const uint64_t bdesc = make_smem_desc_sw128(sa + Cfg::kABytes);
+            for (int i = 0; i < wk.count; ++i) {
+              const uint64_t adesc = make_smem_desc_sw128(sa + i * Cfg::kATile);
+              const uint32_t d = tmem_base + buf * Cfg::kAccCols + i * BLOCK_N;
 #pragma unroll
-          for (int k = 0; k < 4; ++k) umma_f16(d, adesc + 2 * k, bdesc + 2 * k, kIdesc, (kb > 0 || k > 0) ? 1u : 0u);
-          umma_commit(&empty[stage]);
-          if (++stage == kStages) { stage = 0; phase ^= 1u; }
-        }
-        if (!ok) break;
-        umma_commit(&acc_full[buf]);
-        ++acc_iter;
+              for (int k = 0; k < 4; ++k) umma_f16(d, adesc + 2 * k, bdesc + 2 * k, kIdesc, (kb > 0 || k > 0) ? 1u : 0u);
+            }
+            umma_commit(&empty[stage]);
+            if (++stage == kStages) { stage = 0; phase ^= 1u; }
+          }
+          umma_commit(&acc_full[buf]);
+          ++acc_iter;
+          return true;
+        });
       }
     }
   } else if (warp < 2 + kW4ConvWarps) {
@@ -216,46 +248,48 @@ gemm_w4a16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     uint32_t stage = 0, phase = 0, ps = 0, pphase = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-      const int m_tile = item % m_tiles, n_tile = item / m_tiles;
-      const int brow = (p.tile_expert ? p.tile_expert[m_tile] * p.expert_n : 0) + n_tile * BLOCK_N + row;
-      const bool live = brow < p.b_rows && (n_tile * BLOCK_N + row) < p.N;
-      // block scales of this row: 4 bytes per 64-wide slice (2 per thread when two threads share a row)
-      const uint8_t* srow = p.bscale + (size_t)(live ? brow : 0) * p.scale_ld + part * kScaleBytes;
-      auto load_scales = [&](int kb) -> uint32_t {
-        const uint8_t* a = srow + (size_t)kb * 4;
-        return kScaleBytes == 2 ? (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(a)) : (uint32_t)__ldg(a);
-      };
-      uint32_t sc_next = live ? load_scales(0) : 0u;
-      for (int kb = 0; kb < p.k_blocks; ++kb) {
-        const uint32_t sc = sc_next;
-        if (live && kb + 1 < p.k_blocks) sc_next = load_scales(kb + 1);
-        if (!mbar_wait(&p_full[ps], pphase, abort_flag, p.status, 0x720)) { ok = false; break; }
-        const uint32_t* pk = reinterpret_cast<const uint32_t*>(pring + ps * Cfg::kPBytes + row * 32 + part * (kWords * 4));
-        uint32_t w[kWords];
-        if (kWords == 4) {
-          const uint4 v = *reinterpret_cast<const uint4*>(pk);
-          w[0] = v.x; w[1] = v.y; w[2 % kWords] = v.z; w[3 % kWords] = v.w;
-        } else {
-          const uint2 v = *reinterpret_cast<const uint2*>(pk);
-          w[0] = v.x; w[1] = v.y;
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&p_empty[ps]);          // the slice is in registers: its slot can be refilled
-        if (++ps == kPStages) { ps = 0; pphase ^= 1u; }
-        // the operand stage is free once the MMAs that read it last time have retired
-        if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, 0x721)) { ok = false; break; }
-        uint8_t* brow_smem = smem + stage * Cfg::kStageBytes + Cfg::kABytes + (row >> 3) * 1024 + sw * 128;
+      ok = w4_unit<kTiles>(p, item, m_tiles, [&](const W4Work wk) {
+        const int brow = (p.tile_expert ? p.tile_expert[wk.t0] * p.expert_n : 0) + wk.n_tile * BLOCK_N + row;
+        const bool live = brow < p.b_rows && (wk.n_tile * BLOCK_N + row) < p.N;
+        // block scales of this row: 4 bytes per 64-wide slice (2 per thread when two threads share a row)
+        const uint8_t* srow = p.bscale + (size_t)(live ? brow : 0) * p.scale_ld + part * kScaleBytes;
+        auto load_scales = [&](int kb) -> uint32_t {
+          const uint8_t* a = srow + (size_t)kb * 4;
+          return kScaleBytes == 2 ? (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(a)) : (uint32_t)__ldg(a);
+        };
+        uint32_t sc_next = live ? load_scales(0) : 0u;
+        for (int kb = 0; kb < p.k_blocks; ++kb) {
+          const uint32_t sc = sc_next;
+          if (live && kb + 1 < p.k_blocks) sc_next = load_scales(kb + 1);
+          if (!mbar_wait(&p_full[ps], pphase, abort_flag, p.status, 0x720)) return false;
+          const uint32_t* pk = reinterpret_cast<const uint32_t*>(pring + ps * Cfg::kPBytes + row * 32 + part * (kWords * 4));
+          uint32_t w[kWords];
+          if (kWords == 4) {
+            const uint4 v = *reinterpret_cast<const uint4*>(pk);
+            w[0] = v.x; w[1] = v.y; w[2 % kWords] = v.z; w[3 % kWords] = v.w;
+          } else {
+            const uint2 v = *reinterpret_cast<const uint2*>(pk);
+            w[0] = v.x; w[1] = v.y;
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&p_empty[ps]);          // the slice is in registers: its slot can be refilled
+          if (++ps == kPStages) { ps = 0; pphase ^= 1u; }
+          // the operand stage is free once the MMAs that read it last time have retired
+          if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, 0x721)) return false;
+          uint8_t* brow_smem = smem + stage * Cfg::kStageBytes + Cfg::kABytes + (row >> 3) * 1024 + sw * 128;
 #pragma unroll
-        for (int j = 0; j < kWords; ++j) {
-          const __half2 s2 = e4m3_to_half2(sc >> (8 * (j >> 1)));          // one scale per 16 weights = two words
-          const int chunk = part * kWords + j;                             // 16-byte chunk inside the 128-byte row
-          *reinterpret_cast<uint4*>(brow_smem + ((chunk ^ sw) << 4)) = w4_word(w[j], s2);
+          for (int j = 0; j < kWords; ++j) {
+            const __half2 s2 = e4m3_to_half2(sc >> (8 * (j >> 1)));          // one scale per 16 weights = two words
+            const int chunk = part * kWords + j;                             // 16-byte chunk inside the 128-byte row
+            *reinterpret_cast<uint4*>(brow_smem + ((chunk ^ sw) << 4)) = w4_word(w[j], s2);
+          }
+          fence_proxy_async();                 // generic-proxy stores -> visible to the tensor core's async proxy
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&conv[stage]);
+          if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
-        fence_proxy_async();                 // generic-proxy stores -> visible to the tensor core's async proxy
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&conv[stage]);
-        if (++stage == kStages) { stage = 0; phase ^= 1u; }
-      }
+        return true;
+      });
     }
   } else if (warp < 2 + kW4ConvWarps + kW4EpiWarps) {
     // ------------------------------------------------------------------ epilogue
@@ -266,51 +300,56 @@ gemm_w4a16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     uint32_t acc_iter = 0, tile_iter = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
-      const int m_tile = item % m_tiles, n_tile = item / m_tiles;
-      const int m = m_tile * kW4BlockM + row_in_tile;
-      const int brow0 = (p.tile_expert ? p.tile_expert[m_tile] * p.expert_n : 0) + n_tile * BLOCK_N;
-      float* gs = gs_smem + (tile_iter & 1u) * BLOCK_N;
-      ++tile_iter;
-      for (int i = epi_tid; i < BLOCK_N; i += 32 * kW4EpiWarps)
-        gs[i] = (brow0 + i < p.b_rows && n_tile * BLOCK_N + i < p.N) ? __ldg(p.gscale + brow0 + i) : 0.f;
-      asm volatile("bar.sync 1, %0;\n" ::"n"(32 * kW4EpiWarps));
-      if (!ok) continue;
-      const uint32_t buf = acc_iter % kAcc, aph = (acc_iter / kAcc) & 1u;
-      if (!mbar_wait(&acc_full[buf], aph, abort_flag, p.status, 0x730)) { ok = false; continue; }
-      tc_fence_after();
-      const uint32_t taddr = tmem_base + t_lane + buf * BLOCK_N;
-      __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)m * p.ldc;
+      w4_unit<kTiles>(p, item, m_tiles, [&](const W4Work wk) {
+        const int n_tile = wk.n_tile;
+        const int brow0 = (p.tile_expert ? p.tile_expert[wk.t0] * p.expert_n : 0) + n_tile * BLOCK_N;
+        float* gs = gs_smem + (tile_iter & 1u) * BLOCK_N;
+        ++tile_iter;
+        for (int i = epi_tid; i < BLOCK_N; i += 32 * kW4EpiWarps)
+          gs[i] = (brow0 + i < p.b_rows && n_tile * BLOCK_N + i < p.N) ? __ldg(p.gscale + brow0 + i) : 0.f;
+        asm volatile("bar.sync 1, %0;\n" ::"n"(32 * kW4EpiWarps));
+        if (!ok) return true;               // the barrier above counts every warp: the walk goes on
+        const uint32_t buf = acc_iter % kAcc, aph = (acc_iter / kAcc) & 1u;
+        if (!mbar_wait(&acc_full[buf], aph, abort_flag, p.status, 0x730)) { ok = false; return true; }
+        tc_fence_after();
+        for (int i = 0; i < wk.count; ++i) {
+          const int m = (wk.t0 + i) * kW4BlockM + row_in_tile;
+          const uint32_t taddr = tmem_base + t_lane + buf * Cfg::kAccCols + i * BLOCK_N;
+          __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)m * p.ldc;
 #pragma unroll
-      for (int c0 = 0; c0 < BLOCK_N; c0 += 32) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(taddr + c0, r);
-        tmem_ld_wait();
-        if (c0 + 32 >= BLOCK_N) {          // the last chunk is in registers: hand the buffer back
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&acc_empty[buf]);
-        }
-        if (m < M_rows) {
+          for (int c0 = 0; c0 < BLOCK_N; c0 += 32) {
+            uint32_t r[32];
+            tmem_ld_32x32b_x32(taddr + c0, r);
+            tmem_ld_wait();
+            if (i + 1 == wk.count && c0 + 32 >= BLOCK_N) {          // the last chunk is in registers: hand the buffer back
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&acc_empty[buf]);
+            }
+            if (m < M_rows) {
 #pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            const int n = n_tile * BLOCK_N + c0 + j;
-            float v[8];
+              for (int j = 0; j < 32; j += 8) {
+                const int n = n_tile * BLOCK_N + c0 + j;
+                float v[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[j + i]) * gs[c0 + j + i];
-            if (p.vec_ok && n + 8 <= p.N) {
-              uint4 o;
-              o.x = pack_bf16x2(v[0], v[1]); o.y = pack_bf16x2(v[2], v[3]);
-              o.z = pack_bf16x2(v[4], v[5]); o.w = pack_bf16x2(v[6], v[7]);
-              *reinterpret_cast<uint4*>(crow + n) = o;
-            } else {
+                for (int q = 0; q < 8; ++q) v[q] = __uint_as_float(r[j + q]) * gs[c0 + j + q];
+                if (p.vec_ok && n + 8 <= p.N) {
+                  uint4 o;
+                  o.x = pack_bf16x2(v[0], v[1]); o.y = pack_bf16x2(v[2], v[3]);
+                  o.z = pack_bf16x2(v[4], v[5]); o.w = pack_bf16x2(v[6], v[7]);
+                  *reinterpret_cast<uint4*>(crow + n) = o;
+                } else {
 #pragma unroll
-              for (int i = 0; i < 8; ++i)
-                if (n + i < p.N) crow[n + i] = __float2bfloat16_rn(v[i]);
+                  for (int q = 0; q < 8; ++q)
+                    if (n + q < p.N) crow[n + q] = __float2bfloat16_rn(v[q]);
+                }
+              }
             }
           }
         }
-      }
-      ++acc_iter;
+        ++acc_iter;
+        return true;
+      });
     }
   }
 
@@ -322,10 +361,10 @@ gemm_w4a16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   }
 }
 
-template <int BLOCK_N>
+template <int BLOCK_N, int ROWS>
 static int launch_w4(const CUtensorMap& ta, const CUtensorMap& tp, const W4Params& p, int grid, cudaStream_t st) {
-  using Cfg = W4Cfg<BLOCK_N>;
-  auto kern = gemm_w4a16_tcgen05_kernel<BLOCK_N>;
+  using Cfg = W4Cfg<BLOCK_N, ROWS>;
+  auto kern = gemm_w4a16_tcgen05_kernel<BLOCK_N, ROWS>;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), Cfg::kSmemBytes) != cudaSuccess) return -20;
   kern<<<grid, kW4Threads, Cfg::kSmemBytes, st>>>(ta, tp, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
@@ -333,7 +372,7 @@ static int launch_w4(const CUtensorMap& ta, const CUtensorMap& tp, const W4Param
 
 static int w4_common(const void* A, const void* packed, const void* bscale, const float* gscale, void* C, int M, int N,
                      int K, long long lda, long long ldc, int block_n, int b_rows, const int* tile_expert,
-                     const int* num_m_tiles, int num_sms, unsigned long long* status, void* stream) {
+                     const int* unit_tile, const int* num_m_tiles, int rows_hint, int num_sms, unsigned long long* status, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (K % 64) return -3;                                  // one slice = 64 weights = 4 block scales
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(packed) & 15)) return -1;
@@ -353,11 +392,14 @@ static int w4_common(const void* A, const void* packed, const void* bscale, cons
   p.n_tiles = (N + block_n - 1) / block_n;
   p.scale_ld = K / 16; p.b_rows = b_rows;
   p.vec_ok = ((ldc % 8) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) ? 1 : 0;
-  p.tile_expert = tile_expert; p.num_m_tiles_ptr = num_m_tiles; p.expert_n = tile_expert ? N : 0;
-  const long long items = (long long)p.m_tiles * p.n_tiles;
+  p.tile_expert = tile_expert; p.unit_tile = unit_tile; p.num_m_tiles_ptr = num_m_tiles; p.expert_n = tile_expert ? N : 0;
+  // two row tiles a unit where there are two (of an expert, on average) and the units still fill the SMs
+  const bool dual = block_n == 128 && rows_hint > kW4BlockM && (!tile_expert || unit_tile) && (long long)((p.m_tiles + 1) / 2) * p.n_tiles >= num_sms;
+  const long long items = (long long)(dual ? (p.m_tiles + 1) / 2 : p.m_tiles) * p.n_tiles;
   const int grid = (int)(items < num_sms ? items : num_sms);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  return block_n == 64 ? launch_w4<64>(ta, tp, p, grid, st) : launch_w4<128>(ta, tp, p, grid, st);
+  if (dual) return launch_w4<128, 256>(ta, tp, p, grid, st);
+  return block_n == 64 ? launch_w4<64, 128>(ta, tp, p, grid, st) : launch_w4<128, 128>(ta, tp, p, grid, st);
 }
 
 }  // namespace atlas
@@ -369,17 +411,18 @@ using namespace atlas;
 extern "C" int atlas_gemm_w4a16(const void* A, const void* packed, const void* bscale, const float* gscale, void* C,
                                 int M, int N, int K, long long lda, long long ldc, int block_n, int num_sms,
                                 unsigned long long* status, void* stream) {
-  return w4_common(A, packed, bscale, gscale, C, M, N, K, lda, ldc, block_n, N, nullptr, nullptr, num_sms, status, stream);
+  return w4_common(A, packed, bscale, gscale, C, M, N, K, lda, ldc, block_n, N, nullptr, nullptr, nullptr, M, num_sms, status, stream);
 }
 
 // Grouped (MoE) form: rows of A are expert-sorted, every expert's segment padded to whole 128-row tiles; m-tile i uses
 // expert tile_expert[i]; *num_m_tiles (device memory) tiles are live.  packed / bscale / gscale are the stacks over
-// E experts ([E*N, K/2], [E*N, K/16], [E*N]).
+// E experts ([E*N, K/2], [E*N, K/16], [E*N]).  unit_tile, num_m_tiles[1]: see moe_align.
+// rows_hint: rows an expert gets on average.
 extern "C" int atlas_gemm_w4a16_grouped(const void* A, const void* packed, const void* bscale, const float* gscale,
                                         void* C, int max_rows, int N, int K, int E, long long lda, long long ldc,
-                                        int block_n, const int* tile_expert, const int* num_m_tiles, int num_sms,
-                                        unsigned long long* status, void* stream) {
+                                        int block_n, const int* tile_expert, const int* unit_tile, const int* num_m_tiles,
+                                        int rows_hint, int num_sms, unsigned long long* status, void* stream) {
   if (max_rows % kW4BlockM) return -9;
-  return w4_common(A, packed, bscale, gscale, C, max_rows, N, K, lda, ldc, block_n, E * N, tile_expert, num_m_tiles,
-                   num_sms, status, stream);
+  return w4_common(A, packed, bscale, gscale, C, max_rows, N, K, lda, ldc, block_n, E * N, tile_expert, unit_tile, num_m_tiles,
+                   rows_hint, num_sms, status, stream);
 }

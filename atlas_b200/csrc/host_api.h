@@ -66,7 +66,7 @@ int atlas_moe_route_ex(const void* logits, long long ld, int is_bf16, int T, int
                        const float* sel_bias, int n_group, int topk_group, const int* hash_table, const int* token_ids,
                        float out_scale, float* w_out, int* id_out, void* stream);
 int atlas_moe_align(const int* topk_ids, int T, int k, int e_lo, int E_local, int* slot_of, int* row_token,
-                    int* tile_expert, int* tile_rows, int* num_tiles, int max_rows, unsigned long long* status, void* stream);
+                    int* tile_expert, int* tile_rows, int* unit_tile, int* num_tiles, int max_rows, unsigned long long* status, void* stream);
 int atlas_moe_gather(const void* x, long long ldx, const int* slot_of, int T, int k, int H, void* y, void* q, float* scale,
                      long long scale_ld, void* stream);
 int atlas_moe_combine(const void* y, long long ldy, const int* slot_of, const float* topk_w, int T, int k, int H,
@@ -82,8 +82,8 @@ int atlas_gemm_w4a16(const void* A, const void* packed, const void* bscale, cons
                      void* stream);
 int atlas_gemm_w4a16_grouped(const void* A, const void* packed, const void* bscale, const float* gscale, void* C,
                              int max_rows, int N, int K, int E, long long lda, long long ldc, int block_n,
-                             const int* tile_expert, const int* num_m_tiles, int num_sms, unsigned long long* status,
-                             void* stream);
+                             const int* tile_expert, const int* unit_tile, const int* num_m_tiles, int rows_hint, int num_sms,
+                             unsigned long long* status, void* stream);
 int atlas_gemm_grouped(int kind, const void* A, const void* B, void* C, const float* a_scale, long long sa_k,
                        const float* b_scale, int max_rows, int N, int K, int E, long long lda, long long ldb,
                        long long ldc, int block_n, const int* tile_expert, const int* tile_rows, const int* num_m_tiles,

@@ -185,9 +185,10 @@ moe_route_kernel(const T* __restrict__ logits, long long ld, int T_, int E, int 
 // A cluster of 1 or 8 CTAs of 1024 threads; counts and offsets live in shared memory (E <= 1024), every CTA counts and places its
 // share of the pairs and reads the others' counts from their shared memory.
 // slot_of[t*k+j] = row in the expert-sorted buffer, or -1 for experts outside [e_lo, e_lo + E_local).
-// The per-expert tile counts are prefix-summed by the whole block (one expert per thread, log-step scan).  A pair whose
+// The per-expert tile counts are prefix-summed by the whole block (one expert per thread).  A pair whose
 // row would fall beyond max_rows is dropped and recorded as a bounds error in the status word.  tile_rows[i] = live rows
-// of tile i, its leading ones; row_token is written for the rows of live tiles only.
+// of tile i, its leading ones; row_token is written for the rows of live tiles only.  unit_tile (may be null): the first tile of every pair
+// of tiles of one expert (the last of an odd number alone), num_tiles[1] of them.
 // Bound by the latency of loads and shared-memory atomics: ids come four to a load where the list allows it, and only the padding of the
 // live tiles is filled.  8192 tokens x 10 of 512 experts: 66 us with one CTA, 15 us; steps of few pairs stay with one CTA.
 constexpr int kAlignCluster = 8, kAlignClusterPairs = 4096;
@@ -198,13 +199,13 @@ __device__ __forceinline__ int ld_cluster_s32(uint32_t addr) {
 }
 __global__ void __launch_bounds__(1024)
 moe_align_kernel(const int* __restrict__ topk_ids, int n_pairs, int e_lo, int E_local, int* __restrict__ slot_of,
-                 int* __restrict__ row_token, int* __restrict__ tile_expert, int* __restrict__ tile_rows, int* __restrict__ num_tiles,
-                 int max_rows, int k, status_t* status) {
+                 int* __restrict__ row_token, int* __restrict__ tile_expert, int* __restrict__ tile_rows, int* __restrict__ unit_tile,
+                 int* __restrict__ num_tiles, int max_rows, int k, status_t* status) {
   chain_trigger();
   chain_wait();
   __shared__ int mine[1024];                  // this CTA's pairs of an expert
   __shared__ int counts[1024];                // everybody's
-  __shared__ int scan[2][1024];
+  __shared__ int scan[1024], warp_tiles[32];
   __shared__ int cursor[1024];
   const int tid = threadIdx.x, rank = blockIdx.x, ctas = gridDim.x;
   mine[tid] = 0;
@@ -236,16 +237,21 @@ moe_align_kernel(const int* __restrict__ topk_ids, int n_pairs, int e_lo, int E_
   counts[tid] = total;
   cursor[tid] = before;
   const int my_tiles = tid < E_local ? (total + 127) >> 7 : 0;
-  int cur = 0;
-  scan[0][tid] = my_tiles;
-  __syncthreads();
-  for (int d = 1; d < 1024; d <<= 1) {
-    const int v = scan[cur][tid] + (tid >= d ? scan[cur][tid - d] : 0);
-    scan[cur ^ 1][tid] = v;
-    cur ^= 1;
+  auto prefix = [&](int v) {                  // inclusive, over the block: inside the warp, then over the warps' sums
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, v, d);
+      if ((tid & 31) >= d) v += u;
+    }
+    if ((tid & 31) == 31) warp_tiles[tid >> 5] = v;
     __syncthreads();
-  }
-  const int tile0 = scan[cur][tid] - my_tiles;        // exclusive prefix = first tile of this expert
+    v += __reduce_add_sync(0xffffffffu, (tid & 31) < (tid >> 5) ? warp_tiles[tid & 31] : 0);
+    __syncthreads();
+    return v;
+  };
+  scan[tid] = prefix(my_tiles);
+  __syncthreads();
+  const int tile0 = scan[tid] - my_tiles;        // exclusive prefix = first tile of this expert
   const int max_tiles = max_rows >> 7;
   if (rank == 0) {
     for (int i = 0; i < my_tiles; ++i)
@@ -254,13 +260,19 @@ moe_align_kernel(const int* __restrict__ topk_ids, int n_pairs, int e_lo, int E_
         tile_rows[tile0 + i] = min(128, total - 128 * i);
       }
     if (tid == 1023) {
-      const int tiles = scan[cur][1023];
+      const int tiles = scan[1023];
       if (tiles > max_tiles) report_status(status, kBoundsError, 0x700);
       *num_tiles = min(tiles, max_tiles);
     }
+    if (unit_tile != nullptr) {
+      const int my_units = (my_tiles + 1) >> 1, units = prefix(my_units);
+      for (int i = 0; i < my_units; ++i)
+        if (tile0 + 2 * i < max_tiles) unit_tile[units - my_units + i] = tile0 + 2 * i;
+      if (tid == 1023) num_tiles[1] = scan[1023] <= max_tiles ? units : 0;
+    }
   }
   for (int e = rank * 32 + (tid >> 5); e < E_local; e += ctas * 32) {       // a warp per expert: the padding behind its rows
-    const int tiles = (counts[e] + 127) >> 7, base = (scan[cur][e] - tiles) << 7;
+    const int tiles = (counts[e] + 127) >> 7, base = (scan[e] - tiles) << 7;
     for (int r = base + counts[e] + (tid & 31); r < min(base + (tiles << 7), max_rows); r += 32) row_token[r] = -1;
   }
   // Rank inside an expert: pairs are visited in index order by a fixed thread, but threads race on the cursor;
@@ -269,7 +281,7 @@ moe_align_kernel(const int* __restrict__ topk_ids, int n_pairs, int e_lo, int E_
     const int e = id - e_lo;
     int slot = -1;
     if (e >= 0 && e < E_local) {
-      slot = ((scan[cur][e] - ((counts[e] + 127) >> 7)) << 7) + atomicAdd(&cursor[e], 1);
+      slot = ((scan[e] - ((counts[e] + 127) >> 7)) << 7) + atomicAdd(&cursor[e], 1);
       if (slot < max_rows) row_token[slot] = i / k;
       else { slot = -1; report_status(status, kBoundsError, 0x701); }
     }
@@ -520,17 +532,17 @@ extern "C" int atlas_moe_route_ex(const void* logits, long long ld, int is_bf16,
 }
 
 extern "C" int atlas_moe_align(const int* topk_ids, int T, int k, int e_lo, int E_local, int* slot_of, int* row_token,
-                               int* tile_expert, int* tile_rows, int* num_tiles, int max_rows, unsigned long long* status,
-                               void* stream) {
+                               int* tile_expert, int* tile_rows, int* unit_tile, int* num_tiles, int max_rows,
+                               unsigned long long* status, void* stream) {
   if (E_local > 1024 || max_rows % 128) return -1;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int n = T * k;
   if (n < kAlignClusterPairs)
     launch_chain(moe_align_kernel, dim3(1), dim3(1024), 0, st, topk_ids, n, e_lo, E_local, slot_of, row_token, tile_expert, tile_rows,
-                 num_tiles, max_rows, k, status);
+                 unit_tile, num_tiles, max_rows, k, status);
   else
     launch_chain_cluster(false, kAlignCluster, moe_align_kernel, dim3(kAlignCluster), dim3(1024), 0, st, topk_ids, n, e_lo, E_local, slot_of,
-                         row_token, tile_expert, tile_rows, num_tiles, max_rows, k, status);
+                         row_token, tile_expert, tile_rows, unit_tile, num_tiles, max_rows, k, status);
   return cudaGetLastError() == cudaSuccess ? 0 : -20;
 }
 

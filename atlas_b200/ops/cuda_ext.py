@@ -15,7 +15,7 @@ FP8 = torch.float8_e4m3fn
 
 def bind(lib) -> None:
     lib.atlas_moe_route.argtypes = [_vp, _ll, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp]
-    lib.atlas_moe_align.argtypes = [_vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp, _vp]
+    lib.atlas_moe_align.argtypes = [_vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _vp, _vp]
     lib.atlas_moe_gather.argtypes = [_vp, _ll, _vp, _i, _i, _i, _vp, _vp, _vp, _ll, _vp]
     lib.atlas_moe_combine.argtypes = [_vp, _ll, _vp, _vp, _i, _i, _i, _vp, _ll, _vp, _ll, _vp]
     lib.atlas_gemm_grouped.argtypes = [_i, _vp, _vp, _vp, _vp, _ll, _vp, _i, _i, _i, _i, _ll, _ll, _ll, _i, _vp, _vp, _vp, _i, _i, _vp, _vp, _i, _f, _f, _f]
@@ -25,7 +25,7 @@ def bind(lib) -> None:
     lib.atlas_moe_dispatch_pack.argtypes = [_vp, _ll, _vp, _vp, _i, _i, _i, _vp, _i, _vp]
     lib.atlas_moe_recv_ids.argtypes = [_vp, _i, _i, _vp, _i, _i, _vp, _vp]
     lib.atlas_gemm_w4a16.argtypes = [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _ll, _ll, _i, _i, _vp, _vp]
-    lib.atlas_gemm_w4a16_grouped.argtypes = [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _ll, _ll, _i, _vp, _vp, _i, _vp, _vp]
+    lib.atlas_gemm_w4a16_grouped.argtypes = [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _ll, _ll, _i, _vp, _vp, _vp, _i, _i, _vp, _vp]
     for name, args in _GDN_SIGS.items():
         if hasattr(lib, name):
             getattr(lib, name).argtypes = args
@@ -311,10 +311,11 @@ def _moe_local(x, topk_w, topk_ids, experts, e_lo, addend: Optional[torch.Tensor
     lib, st, sms, status = K.lib(), K._stream(), K._num_sms[d], K._status_ptr[d]
     slot_of = torch.empty(T * k, dtype=torch.int32, device=dev)
     row_token = torch.empty(max_rows, dtype=torch.int32, device=dev)
-    tile_expert, tile_rows = torch.empty(2, max_tiles, dtype=torch.int32, device=dev)
-    num_tiles = torch.empty(1, dtype=torch.int32, device=dev)
+    tile_expert, tile_rows, unit_tile = torch.empty(3, max_tiles, dtype=torch.int32, device=dev)
+    num_tiles = torch.empty(2, dtype=torch.int32, device=dev)
     K._check(lib.atlas_moe_align(topk_ids.data_ptr(), T, k, e_lo, E, slot_of.data_ptr(), row_token.data_ptr(),
-                                 tile_expert.data_ptr(), tile_rows.data_ptr(), num_tiles.data_ptr(), max_rows, status, st), "moe_align")
+                                 tile_expert.data_ptr(), tile_rows.data_ptr(), unit_tile.data_ptr() if kind == 2 else None, num_tiles.data_ptr(), max_rows,
+                                 status, st), "moe_align")
 
     def bn_for(n):
         return 128 if n % 128 == 0 else 64
@@ -360,8 +361,8 @@ def _moe_local(x, topk_w, topk_ids, experts, e_lo, addend: Optional[torch.Tensor
     h1 = torch.empty(max_rows, N1o, dtype=torch.bfloat16, device=dev)
     if kind == 2:
         K._check(lib.atlas_gemm_w4a16_grouped(a1.data_ptr(), w13.data_ptr(), s13[0].data_ptr(), s13[1].data_ptr(), h1.data_ptr(),
-                                              max_rows, N1, H, E, H, N1, bn_for(N1), tile_expert.data_ptr(),
-                                              num_tiles.data_ptr(), sms, status, st), "moe_gemm1_w4")
+                                              max_rows, N1, H, E, H, N1, bn_for(N1), tile_expert.data_ptr(), unit_tile.data_ptr(),
+                                              num_tiles.data_ptr(), T * k // E, sms, status, st), "moe_gemm1_w4")
     else:
         K._check(lib.atlas_gemm_grouped(kind, a1.data_ptr(), w13.data_ptr(), h1.data_ptr(), K._ptr(a1s), max_rows, K._ptr(s13),
                                         max_rows, N1, H, E, H, H, N1o, bn_for(N1), tile_expert.data_ptr(),
@@ -383,8 +384,8 @@ def _moe_local(x, topk_w, topk_ids, experts, e_lo, addend: Optional[torch.Tensor
     y = torch.empty(max_rows, H, dtype=torch.bfloat16, device=dev)
     if kind == 2:
         K._check(lib.atlas_gemm_w4a16_grouped(a2.data_ptr(), w2.data_ptr(), s2[0].data_ptr(), s2[1].data_ptr(), y.data_ptr(),
-                                              max_rows, H, I, E, I, H, bn_for(H), tile_expert.data_ptr(), num_tiles.data_ptr(),
-                                              sms, status, st), "moe_gemm2_w4")
+                                              max_rows, H, I, E, I, H, bn_for(H), tile_expert.data_ptr(), unit_tile.data_ptr(), num_tiles.data_ptr(),
+                                              T * k // E, sms, status, st), "moe_gemm2_w4")
     else:
         K._check(lib.atlas_gemm_grouped(kind, a2.data_ptr(), w2.data_ptr(), y.data_ptr(), K._ptr(a2s), max_rows, K._ptr(s2),
                                         max_rows, H, I, E, I, I, H, bn_for(H), tile_expert.data_ptr(),

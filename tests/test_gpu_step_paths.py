@@ -80,10 +80,10 @@ def test_expert_row_lists(K, T, k):
     ids = torch.stack([torch.randperm(E)[:k] for _ in range(T)]).int().to(DEV)
     tiles = T * k // 128 + min(T * k, n)
     slot, rows = torch.empty(T * k, dtype=torch.int32, device=DEV), torch.full((tiles * 128,), -7, dtype=torch.int32, device=DEV)
-    te, tr, nt = (torch.zeros(m, dtype=torch.int32, device=DEV) for m in (tiles, tiles, 1))
-    K._check(K.lib().atlas_moe_align(ids.data_ptr(), T, k, lo, n, slot.data_ptr(), rows.data_ptr(), te.data_ptr(), tr.data_ptr(), nt.data_ptr(),
+    te, tr, un, nt = (torch.zeros(m, dtype=torch.int32, device=DEV) for m in (tiles, tiles, tiles, 2))
+    K._check(K.lib().atlas_moe_align(ids.data_ptr(), T, k, lo, n, slot.data_ptr(), rows.data_ptr(), te.data_ptr(), tr.data_ptr(), un.data_ptr(), nt.data_ptr(),
                                      tiles * 128, K._status_ptr[K._dev(ids)], K._stream()), "moe_align")
-    live = int(nt)
+    live, units = nt.tolist()
     assert int(tr[:live].sum()) == int(((ids >= lo) & (ids < lo + n)).sum())
     flat, slot, te, tr, rows = ids.flatten().tolist(), slot.tolist(), te.tolist(), tr.tolist(), rows.tolist()
     used = [s for s in slot if s >= 0]
@@ -92,6 +92,12 @@ def test_expert_row_lists(K, T, k):
         assert (s >= 0) == (lo <= e < lo + n)
         if s >= 0:
             assert te[s // 128] == e - lo and s % 128 < tr[s // 128] and rows[s] == i // k
+    left, starts = list(range(live)), un[:units].tolist()             # units: pairs of tiles of one expert from its first on
+    for t in starts:
+        left.remove(t)
+        if t + 1 < live and te[t + 1] == te[t]:
+            left.remove(t + 1)
+    assert not left
     for t in range(live):
         assert all(r == -1 for r in rows[t * 128 + tr[t]:(t + 1) * 128])
 
