@@ -180,7 +180,7 @@ int atlas_tanh(void* x, long long n, int f32, void* stream);
 int atlas_mamba2_scan(const void* y, long long ldy, const void* dt, long long lddt, const float* A_log, const float* D,
                       const float* dt_bias, float dt_min, float* h, void* out, long long ldo, const int* qsl, const int* slots,
                       const unsigned char* has, const int* limit, const int* snap_rows, const int* snap_slots, int snaps, int B, int H,
-                      int P, int N, int G, int commit, int one_row, int longest, int shortest, int f32, void* stream);
+                      int P, int N, int G, int commit, int one_row, int f32, void* stream);
 int atlas_wkv_scan(const void* r, long long ldr, const void* k, long long ldk, const void* v, long long ldv, const void* raw, long long ldw,
                    const float* w0, const float* u, float* h, void* out, long long ldo, const void* x, long long ldx, void* shift, int W,
                    const int* qsl, const int* slots, const unsigned char* has, const int* limit, const int* snap_rows,

@@ -47,7 +47,6 @@ struct ScanParams {
   const int* query_start_loc; const int* state_slots; const unsigned char* has_state; const int* limit;
   const int* snap_rows; const int* snap_slots; int num_snaps_per_seq;
   int H, P, N, G, commit;
-  int row_hi;                                  // sequences of as many rows or more are another launch's (0 = none)
 };
 
 constexpr int kScanRows = 16, kGroup = 4;
@@ -136,7 +135,7 @@ linear_scan_kernel(const ScanParams<T> p) {
   const int q0 = p.query_start_loc[bseq];
   const int qlen = p.query_start_loc[bseq + 1] - q0;
   const int n_rows = p.limit ? min(p.limit[bseq], qlen) : qlen;
-  if (n_rows <= 0 || (p.row_hi > 0 && n_rows >= p.row_hi)) return;
+  if (n_rows <= 0) return;
   const long long slot = p.state_slots[bseq];
   const bool walker = threadIdx.x < 128;
   const int tid = threadIdx.x & 127, warp = tid >> 5, lane = tid & 31;

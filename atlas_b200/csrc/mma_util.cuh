@@ -37,15 +37,4 @@ ATLAS_DEVICE void split_bf16x2(float a, float b, uint32_t& hi, uint32_t& lo) {
   lo = pack_bf16x2(a - f.x, b - f.y);
 }
 
-// fp32 pair as three bf16 terms each
-ATLAS_DEVICE void split3_bf16x2(float a, float b, uint32_t (&t)[3]) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    const float2 f = __bfloat1622float2(h);
-    t[i] = *reinterpret_cast<const uint32_t*>(&h);
-    a -= f.x; b -= f.y;
-  }
-}
-
 }  // namespace atlas

@@ -1,11 +1,8 @@
 // Mamba-2 and WKV recurrences (kernels in linear_scan.cuh).  Activations are bf16 or fp32 (template parameter T).
 // Reference ops replaced: kernels/gb10/common/mamba2_ssm_decode.cu, mamba2_ssd_chunk.cu.
-#include <type_traits>
-
 #include "common.cuh"
 #include "host_api.h"
 #include "linear_scan.cuh"
-#include "mamba2_chunk.cuh"
 #include "vec_io.cuh"
 
 namespace atlas {
@@ -14,18 +11,11 @@ template <typename T>
 static int mamba2(const void* y, long long ldy, const void* dt, long long lddt, const float* A_log, const float* D,
                   const float* dt_bias, float dt_min, float* h, void* out, long long ldo, const int* qsl, const int* slots,
                   const unsigned char* has, const int* limit, const int* snap_rows, const int* snap_slots, int snaps, int B, int H,
-                  int P, int N, int G, int commit, int one_row, int longest, int shortest, cudaStream_t st) {
+                  int P, int N, int G, int commit, int one_row, cudaStream_t st) {
   ScanParams<T> p = {};
   p.a = reinterpret_cast<const T*>(y); p.lda = ldy; p.b = reinterpret_cast<const T*>(dt); p.ldb = lddt;
   p.A_log = A_log; p.D = D; p.dt_bias = dt_bias; p.dt_min = dt_min;
   fill_batch(p, h, out, ldo, qsl, slots, has, limit, snap_rows, snap_slots, snaps, H, P, N, G, commit);
-  if constexpr (std::is_same_v<T, __nv_bfloat16>) {
-    if (longest >= 2 * kMcMin) {             // prefill steps
-      const int rc = mamba2_chunked(p, B, st);
-      if (rc < 0 || (rc == 0 && shortest >= kMcMin)) return rc;
-      if (rc == 0) p.row_hi = kMcMin;
-    }
-  }
   return scan<T, kMamba>(p, B, one_row, st);
 }
 
@@ -47,17 +37,16 @@ static int wkv(const void* r, long long ldr, const void* k, long long ldk, const
 using namespace atlas;
 using bf16 = __nv_bfloat16;
 
-// longest, shortest: rows of the step's longest and shortest sequence
 extern "C" int atlas_mamba2_scan(const void* y, long long ldy, const void* dt, long long lddt, const float* A_log, const float* D,
                                  const float* dt_bias, float dt_min, float* h, void* out, long long ldo, const int* qsl,
                                  const int* slots, const unsigned char* has, const int* limit, const int* snap_rows,
-                                 const int* snap_slots, int snaps, int B, int H, int P, int N, int G, int commit, int one_row, int longest,
-                                 int shortest, int f32, void* stream) {
+                                 const int* snap_slots, int snaps, int B, int H, int P, int N, int G, int commit, int one_row, int f32,
+                                 void* stream) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   return f32 ? mamba2<float>(y, ldy, dt, lddt, A_log, D, dt_bias, dt_min, h, out, ldo, qsl, slots, has, limit, snap_rows, snap_slots, snaps,
-                             B, H, P, N, G, commit, one_row, longest, shortest, st)
+                             B, H, P, N, G, commit, one_row, st)
              : mamba2<bf16>(y, ldy, dt, lddt, A_log, D, dt_bias, dt_min, h, out, ldo, qsl, slots, has, limit, snap_rows, snap_slots, snaps,
-                            B, H, P, N, G, commit, one_row, longest, shortest, st);
+                            B, H, P, N, G, commit, one_row, st);
 }
 
 // r may be null: the state is advanced and nothing is written to `out` (write-on-accept fold)

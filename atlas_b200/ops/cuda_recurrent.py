@@ -39,7 +39,7 @@ def _lib():
         lib.atlas_rglru_scan.argtypes = [C.POINTER(_Rglru), _i, _vp]
         lib.atlas_row_norm_kv_write.argtypes = [_vp, _ll, _vp, _ll, _vp, _ll] + [_vp] * 9 + [_i] * 8 + [_f, _f, _i, _i, _vp]
         lib.atlas_tanh.argtypes = [_vp, _ll, _i, _vp]
-        lib.atlas_mamba2_scan.argtypes = [_vp, _ll, _vp, _ll, _vp, _vp, _vp, _f, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _vp] + [_i] * 11 + [_vp]
+        lib.atlas_mamba2_scan.argtypes = [_vp, _ll, _vp, _ll, _vp, _vp, _vp, _f, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _vp] + [_i] * 9 + [_vp]
         lib.atlas_wkv_scan.argtypes = [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _ll, _vp, _vp, _vp, _vp, _ll, _vp, _ll, _vp, _i, _vp, _vp, _vp,
                                        _vp, _vp, _vp] + [_i] * 7 + [_vp]
         lib.atlas_group_norm_gate.argtypes = [_vp, _ll, _vp, _ll, _vp, _vp, _ll, _i, _i, _i, _f, _i, _i, _vp, _i, _vp]
@@ -172,8 +172,7 @@ def _mamba2_run(layer, xbc, dt, meta: _Meta, state, commit: bool):
                                    layer.dt_bias.data_ptr(), float(layer.cfg.mamba_dt_min), h.data_ptr(), out.data_ptr(),
                                    layer.d_inner, meta.qsl.data_ptr(), meta.slots.data_ptr(), meta.has.data_ptr(),
                                    K._ptr(meta.limit), meta.snap_rows.data_ptr(), meta.snap_slots.data_ptr(), meta.snaps, meta.B,
-                                   layer.h, layer.p, layer.n, layer.g, 1 if commit else 0, meta.one_row, meta.longest, meta.shortest, f32, st),
-             "mamba2_scan")
+                                   layer.h, layer.p, layer.n, layer.g, 1 if commit else 0, meta.one_row, f32, st), "mamba2_scan")
     conv_advance(xbc, layer.W, conv, meta, commit)
     return out
 

@@ -259,55 +259,6 @@ def test_chunked_delta_rule_workspace_is_bounded(K):
     assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
 
 
-# ----------------------------------------------------------------------------- chunked Mamba-2
-def _mamba_scan(u, dt, a_log, skip, bias, h, H, G, stops):
-    """The recurrence in 64 bits over rows [x | B | C]: outputs, and the state after every row count in ``stops``."""
-    n, P, N = u.shape[0], 64, 128
-    u, h, kept, out = u.double(), h.double().clone(), {}, []
-    x, b, c = u[:, :H * P].view(n, H, P), u[:, H * P:H * P + G * N].view(n, G, N), u[:, H * P + G * N:].view(n, G, N)
-    b, c = b.repeat_interleave(H // G, 1), c.repeat_interleave(H // G, 1)
-    step = torch.nn.functional.softplus(dt.double() + bias.double()).clamp_min(1e-4)
-    decay = torch.exp(-torch.exp(a_log.double()) * step)
-    for t in range(n):
-        h = h * decay[t][:, None, None] + (step[t][:, None] * x[t])[:, :, None] * b[t][:, None, :]
-        out.append((torch.einsum("hpn,hn->hp", h, c[t]) + skip.double()[:, None] * x[t]).flatten())
-        if t + 1 in stops:
-            kept[t + 1] = h.clone()
-    return torch.stack(out), kept
-
-
-@pytest.mark.parametrize("lens,snaps", [([64, 63, 65], {}), ([300, 1, 15, 16, 128], {0: [(1, 6), (64, 7), (200, 8)], 2: [(9, 9)], 4: [(128, 10)]}), ([1100], {})])
-def test_chunked_mamba2_against_64_bits(K, lens, snaps):
-    """Edges of the 64-row chunks, snapshot rows inside and on them, sequences that stay with the row-by-row kernel, and heads from slow
-    to fast decays.  States are fp32 sums of operands in 24 bits: no worse than the row-by-row kernel's (its rounding of the whole
-    state at every row), and 1e-6 in any case; outputs are rounded to bf16."""
-    from atlas_b200.ops import cuda_gdn, cuda_recurrent as R
-    torch.manual_seed(sum(lens))
-    H, G, P, N, T, B = 8, 2, 64, 128, sum(lens), len(lens)
-    u = torch.randn(T, H * P + 2 * G * N, device=DEV).bfloat16()
-    dt = torch.randn(T, H, device=DEV).bfloat16()
-    a_log, bias = torch.linspace(-3, 3, H, device=DEV), torch.tensor([-6.0, -4.0, -2.0, 0.0, 1.0, 1.0, -6.0, -4.0], device=DEV)
-    skip, h0 = torch.randn(H, device=DEV), torch.randn(12, H, P, N, device=DEV)
-    has = [i % 2 == 0 for i in range(B)]
-    meta, res = cuda_gdn._Meta(lens, list(range(B)), has, DEV, snaps), []
-    for longest in (meta.longest, 0):                          # chunked; row by row
-        h, out = h0.clone(), torch.empty(T, H * P, dtype=torch.bfloat16, device=DEV)
-        K._check(R._lib().atlas_mamba2_scan(u.data_ptr(), u.stride(0), dt.data_ptr(), H, a_log.data_ptr(), skip.data_ptr(), bias.data_ptr(), 1e-4, h.data_ptr(),
-                                            out.data_ptr(), H * P, meta.qsl.data_ptr(), meta.slots.data_ptr(), meta.has.data_ptr(), None,
-                                            meta.snap_rows.data_ptr(), meta.snap_slots.data_ptr(), meta.snaps, B, H, P, N, G, 1, 0, longest,
-                                            meta.shortest, 0, K._stream()), "mamba2_scan")
-        res.append((out, h))
-    t = 0
-    for i, n in enumerate(lens):
-        rows = slice(t, t + n)
-        t += n
-        stops = {r: s for r, s in snaps.get(i, [])}
-        want, kept = _mamba_scan(u[rows], dt[rows], a_log, skip, bias, h0[i] * has[i], H, G, set(stops) | {n})
-        assert _rel(res[0][0][rows], want) < 2 ** -9
-        for slot, ref64 in [(i, kept[n])] + [(s, kept[r]) for r, s in stops.items()]:
-            assert _rel(res[0][1][slot], ref64) < max(1e-6, _rel(res[1][1][slot], ref64))
-
-
 # ----------------------------------------------------------------------------- chunk attention of 256-wide heads
 @pytest.mark.parametrize("kv", [torch.float8_e4m3fn, torch.bfloat16])
 @pytest.mark.parametrize("Hq,Hkv,qlens,ctxs", [(16, 2, [300, 1, 37, 63], [0, 90, 1000, 77]), (8, 2, [64, 65, 129], [64, 63, 0]), (4, 4, [130, 16], [1, 500]),
