@@ -301,6 +301,7 @@ def _moe_local(x, topk_w, topk_ids, experts, e_lo, addend: Optional[torch.Tensor
     own_act = activation in _EXPERT_ACTS               # not the SwiGLU of the other paths
     E = experts.num_local
     plain = x.dtype == torch.float32 or (experts.kind == "dense" and own_act and (H % 64 or experts.w2.shape[2] % 64))
+    kind = None                                        # experts in fp32 sums: no row tiles, so no pairs of them
     if not plain:
         kind, w13, s13, w2, s2 = _expert_stacks(experts)
         I = w2.shape[2] * 2 if kind == 2 else w2.shape[2]
