@@ -42,11 +42,11 @@ def test_experts_in_fp32_sums(calls, dtype, H, I, activation):
     out = _run(5, 4, H, I, ex, activation, dtype)
     assert out.shape == (5, H) and out.dtype == dtype
     assert [c[0] for c in calls] == ["atlas_moe_align", "atlas_moe_plain_gemm", "atlas_moe_plain_gemm", "atlas_moe_plain_combine"]
-    assert calls[0][1][8] is None
+    assert calls[0][1][9] is None
 
 
 @pytest.mark.parametrize("kind", ["dense", "fp8_block", "nvfp4"])
 def test_only_nvfp4_products_get_pairs_of_tiles(calls, kind):
     ex = ExpertWeights.from_dense(torch.randn(2, 512, 256).bfloat16(), torch.randn(2, 256, 256).bfloat16(), kind)
     _run(40, 2, 256, 256, ex, "silu_glu")
-    assert calls[0][0] == "atlas_moe_align" and (calls[0][1][8] is not None) == (kind == "nvfp4")
+    assert calls[0][0] == "atlas_moe_align" and (calls[0][1][9] is not None) == (kind == "nvfp4")
