@@ -271,9 +271,6 @@ gemm_w4a16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
             const uint2 v = *reinterpret_cast<const uint2*>(pk);
             w[0] = v.x; w[1] = v.y;
           }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&p_empty[ps]);          // the slice is in registers: its slot can be refilled
-          if (++ps == kPStages) { ps = 0; pphase ^= 1u; }
           // the operand stage is free once the MMAs that read it last time have retired
           if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, 0x721)) return false;
           uint8_t* brow_smem = smem + stage * Cfg::kStageBytes + Cfg::kABytes + (row >> 3) * 1024 + sw * 128;
@@ -283,9 +280,13 @@ gemm_w4a16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
             const int chunk = part * kWords + j;                             // 16-byte chunk inside the 128-byte row
             *reinterpret_cast<uint4*>(brow_smem + ((chunk ^ sw) << 4)) = w4_word(w[j], s2);
           }
-          fence_proxy_async();                 // generic-proxy stores -> visible to the tensor core's async proxy
+          // The fence stands between two pairs of proxies: the stores above and the tensor core's reads, the loads of the packed slice and
+          // the copy that refills its slot.  The stores need the loaded values, so the loads are over here.  A slot that was handed back
+          // right behind the loads was now and then refilled under them while the MMAs of two row tiles kept shared memory busy.
+          fence_proxy_async();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&conv[stage]);
+          if (lane == 0) { mbar_arrive(&conv[stage]); mbar_arrive(&p_empty[ps]); }
+          if (++ps == kPStages) { ps = 0; pphase ^= 1u; }
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
         return true;

@@ -145,6 +145,99 @@ def test_silu_rows_share_blocks(K, T, I):
     assert int(q[~got].sum()) == 0 and float(s.t()[~got].abs().sum()) == 0
 
 
+# ----------------------------------------------------------------------------- NVFP4 products of two row tiles a unit
+def _row_lists(K, ids, n):
+    """Row lists of ``n`` experts: (slot of every pair, tile_expert, unit_tile, num_tiles, rows of the buffer)."""
+    T, k = ids.shape
+    tiles = T * k // 128 + min(T * k, n)
+    slot, rows = torch.empty(T * k, dtype=torch.int32, device=DEV), torch.empty(tiles * 128, dtype=torch.int32, device=DEV)
+    te, tr, un, nt = (torch.zeros(m, dtype=torch.int32, device=DEV) for m in (tiles, tiles, tiles, 2))
+    K._check(K.lib().atlas_moe_align(ids.data_ptr(), T, k, 0, n, slot.data_ptr(), rows.data_ptr(), te.data_ptr(), tr.data_ptr(), un.data_ptr(), nt.data_ptr(),
+                                     tiles * 128, K._status_ptr[K._dev(ids)], K._stream()), "moe_align")
+    return slot.long(), te, un, nt, tiles * 128
+
+
+def _nvfp4(g, E, N, H):
+    """Random stack: codes, block scales, a global scale per row."""
+    return (torch.randint(0, 256, (E, N, H // 2), generator=g, device=DEV, dtype=torch.uint8),
+            (torch.rand(E, N, H // 16, generator=g, device=DEV) + 0.5).to(torch.float8_e4m3fn), torch.rand(E * N, generator=g, device=DEV) * 0.02 + 0.005)
+
+
+def _nvfp4_value(w, e, rows):
+    lut = torch.tensor([0, 0.5, 1, 1.5, 2, 3, 4, 6], dtype=torch.float64, device=DEV)
+    lut = torch.cat([lut, -lut])
+    v = torch.stack([lut[(w[0][e] & 15).long()], lut[(w[0][e] >> 4).long()]], -1).flatten(1)
+    return v * w[1][e].double().repeat_interleave(16, 1) * w[2][e * rows:(e + 1) * rows].double()[:, None]
+
+
+def _grouped(K, a, w, N, H, te, un, nt, hint, sms):
+    c = torch.zeros(a.shape[0], N, dtype=torch.bfloat16, device=DEV)
+    E = w[0].shape[0]
+    K._check(K.lib().atlas_gemm_w4a16_grouped(a.data_ptr(), w[0].data_ptr(), w[1].data_ptr(), w[2].data_ptr(), c.data_ptr(), a.shape[0], N, H, E, H, N, 128,
+                                              te.data_ptr(), un.data_ptr(), nt.data_ptr(), hint, sms, K._status_ptr[K._dev(a)], K._stream()), "w4_grouped")
+    return c
+
+
+@pytest.mark.parametrize("counts", [[1, 128, 129, 256], [257, 0, 640, 300], [513, 127, 1, 0], [385]])
+@pytest.mark.parametrize("N,H", [(128, 64), (384, 1088)])
+def test_nvfp4_products_of_two_row_tiles(K, counts, N, H):
+    """Experts with no, one, two, three and five tiles, last tiles of one row: pairs of tiles (``hint`` above 128) against one tile a unit, the
+    same bits on live rows (every accumulator gets the same MMAs in the same order), and against 64 bits (results are rounded to bf16, 2^-9).
+    Eight CTAs walk over all units, so rings and accumulators go round many times."""
+    from atlas_b200.ops import cuda_ext
+    cuda_ext.bind(K.lib())
+    g = torch.Generator(device=DEV).manual_seed(sum(counts) + N)
+    E = len(counts)
+    ids = torch.cat([torch.full((n,), e) for e, n in enumerate(counts)]).int()
+    ids = ids[torch.randperm(len(ids))].to(DEV).view(-1, 1)
+    slot, te, un, nt, rows = _row_lists(K, ids, E)
+    w = _nvfp4(g, E, N, H)
+    a = torch.randn(rows, H, generator=g, device=DEV).bfloat16()
+    one, two = (_grouped(K, a, w, N, H, te, un, nt, hint, 8) for hint in (0, 129))
+    assert K.check_status() == 0
+    assert torch.equal(one[slot], two[slot])
+    for e, n in enumerate(counts):
+        r = slot[ids[:, 0] == e]
+        if n:
+            assert _rel(two[r], a[r].double() @ _nvfp4_value(w, e, N).t()) < 2 ** -9 + 1e-5
+
+
+def test_nvfp4_products_of_two_row_tiles_at_full_rate(K):
+    """Expert products of a large prompt step (the tensor cores then take all of shared memory's bandwidth): the same bits as one tile a
+    unit, in every run."""
+    from atlas_b200.ops import cuda_ext
+    cuda_ext.bind(K.lib())
+    g = torch.Generator(device=DEV).manual_seed(7)
+    E, sms = 128, K._num_sms[K._dev(torch.empty(1, device=DEV))]
+    ids = torch.rand(4500, E, generator=g, device=DEV).topk(8, -1).indices.int().contiguous()
+    slot, te, un, nt, rows = _row_lists(K, ids, E)
+    for N, H in ((1536, 2048), (2048, 768)):
+        w, a = _nvfp4(g, E, N, H), torch.randn(rows, H, generator=g, device=DEV).bfloat16()
+        one = _grouped(K, a, w, N, H, te, un, nt, 0, sms)[slot]
+        for _ in range(8):
+            assert torch.equal(_grouped(K, a, w, N, H, te, un, nt, 281, sms)[slot], one)
+    assert K.check_status() == 0
+
+
+@pytest.mark.parametrize("M,N,Kd,sms", [(257, 128, 64, 2), (300, 200, 192, 4), (512, 136, 2048, 3), (2500, 4096, 1024, 148), (2304, 4032, 512, 148), (1153, 4096, 4096, 148)])
+def test_plain_nvfp4_product_of_two_row_tiles(K, M, N, Kd, sms):
+    """Odd and even tile counts, rows past M, columns past N: pairs of row tiles against one (taken when there are fewer units than SMs)."""
+    from atlas_b200.ops import cuda_ext
+    cuda_ext.bind(K.lib())
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    w = _nvfp4(g, 1, N, Kd)
+    x = torch.randn(M, Kd, generator=g, device=DEV).bfloat16()
+    got = []
+    for s in (sms, 1 << 20):
+        c = torch.zeros(M + 1, N, dtype=torch.bfloat16, device=DEV)
+        K._check(K.lib().atlas_gemm_w4a16(x.data_ptr(), w[0].data_ptr(), w[1].data_ptr(), w[2].data_ptr(), c.data_ptr(), M, N, Kd, Kd, N, 128, s,
+                                          K._status_ptr[K._dev(x)], K._stream()), "w4")
+        got.append(c)
+    assert K.check_status() == 0
+    assert torch.equal(got[0], got[1]) and float(got[0][M].abs().max()) == 0
+    assert _rel(got[0][:M], x.double() @ _nvfp4_value(w, 0, N).t()) < 2 ** -9 + 1e-5
+
+
 # ----------------------------------------------------------------------------- decode graphs of Gated DeltaNet models
 @pytest.mark.parametrize("n", [1, 3, 9])
 def test_delta_net_decode_graph_equals_eager_steps(K, n):
