@@ -126,7 +126,7 @@ struct GemmParams {
   // [21] rows summed.  Nothing is stamped inside the per-slice loops of the epilogue warps: their register budget is
   // what the fold needs.
   unsigned long long* timeline;
-  const int* tile_expert;       // nullptr = plain GEMM
+  const int* tile_expert;       // nullptr = plain GEMM (EXPERTS kernels only)
   const int* tile_rows;         // live rows of every tile, its leading ones: the others are neither copied nor stored
   const int* num_m_tiles_ptr;   // device-side tile count (the host cannot know it)
   int expert_n;                 // output features per expert
@@ -184,14 +184,15 @@ ATLAS_DEVICE uint64_t pack_f32x2(float lo, float hi) {
 
 // Work item -> (m-tile, n-tile, K split).  Cluster mode: consecutive CTAs are the splits of one n-tile.
 struct ItemPos { int m_tile, n_tile, split; };
+template <bool EXPERTS>
 ATLAS_DEVICE ItemPos item_pos(const GemmParams& p, int item, int m_tiles) {
   ItemPos r;
-  if (p.cluster_splits > 1) {
-    r.m_tile = 0; r.n_tile = item / p.cluster_splits; r.split = item % p.cluster_splits;
-  } else if (p.tile_expert != nullptr) {
+  if (EXPERTS) {
     // Experts: the column tiles of a row tile one after the other, so that its rows come from HBM once and from L2 after that (row tiles
     // first read 230 MB of rows again for every column tile: 8192 tokens x 10 of 512 experts, 878 and 844 us a layer).
     r.m_tile = item / p.n_tiles; r.n_tile = item % p.n_tiles; r.split = 0;
+  } else if (p.cluster_splits > 1) {
+    r.m_tile = 0; r.n_tile = item / p.cluster_splits; r.split = item % p.cluster_splits;
   } else {
     r.m_tile = item % m_tiles;
     const int rest = item / m_tiles;
@@ -316,7 +317,9 @@ ATLAS_DEVICE void cluster_tail(const GemmParams& p, uint8_t* smem, const float (
 
 // TRACE compiles the phase stamps of GemmParams::timeline in; the kernels that serve traffic are built without them (a
 // few extra instructions in the single-thread producer / MMA loops were worth 5 % of a prefill-size GEMM).
-template <int BLOCK_N, bool FP8, bool FUSE_AR = false, int EPW = epi_warps(BLOCK_N, FP8), bool TRACE = false>
+// EXPERTS: the grouped form, likewise compiled apart.  As branches on the parameters it cost every plain product: four layers of a dense 8 B
+// FP8 model, 8 x 1024 prompt rows 12660 us, apart 12406; one decode row 480 and 470 us.
+template <int BLOCK_N, bool FP8, bool FUSE_AR = false, int EPW = epi_warps(BLOCK_N, FP8), bool TRACE = false, bool EXPERTS = false>
 __global__ void __launch_bounds__(gemm_threads_w(EPW, FUSE_AR), 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const GemmParams p) {
@@ -383,11 +386,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   // before waiting for that kernel: their HBM latency overlaps its tail.  `pf_*` is a cursor over this CTA's
   // (item, k-slice) sequence that stays p.prefetch_b slices ahead of the ring's loads.
   int pf_item = blockIdx.x, pf_kb = 0, pf_kb1 = 0, pf_row = 0, pf_ahead = 0;
-  const bool pf_on = p.prefetch_b > 0 && p.tile_expert == nullptr;
+  const bool pf_on = !EXPERTS && p.prefetch_b > 0;
   const int pf_total = p.m_tiles * p.n_tiles * p.splits;
   auto pf_enter = [&]() {
     if (pf_item < pf_total) {
-      const ItemPos ip = item_pos(p, pf_item, p.m_tiles);
+      const ItemPos ip = item_pos<false>(p, pf_item, p.m_tiles);
       const int split = ip.split;
       pf_row = ip.n_tile * BLOCK_N;
       pf_kb = split * p.kb_per_split;
@@ -416,9 +419,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   chain_wait();                         // barriers, TMEM and descriptors are set up; global memory from here on
   if (tl && threadIdx.x == 0) tl[3] = clock64();
 
-  const int m_tiles = p.tile_expert ? *p.num_m_tiles_ptr : p.m_tiles;
+  const int m_tiles = EXPERTS ? *p.num_m_tiles_ptr : p.m_tiles;
   const int total_items = m_tiles * p.n_tiles * p.splits;
-  const int M_rows = p.tile_expert ? m_tiles * kBlockM : p.M;
+  const int M_rows = EXPERTS ? m_tiles * kBlockM : p.M;
   const uint32_t ar_epoch = FUSE_AR ? p.ar_state[0] + 1u : 0u;
   uint32_t* const part_flags = FUSE_AR ? p.ar_flags[p.ar_rank] : nullptr;                       // [tile][src]
   (void)part_flags;
@@ -432,7 +435,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     uint32_t seen[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};         // m-tiles known to be complete (up to 256)
     const uint32_t want_epoch = p.a_ready ? *p.a_ready_epoch : 0u;
     for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-      const ItemPos ip = item_pos(p, item, m_tiles);
+      const ItemPos ip = item_pos<EXPERTS>(p, item, m_tiles);
       const int m_tile = ip.m_tile;
       if (p.a_ready != nullptr && !((m_tile < 256) && (seen[m_tile >> 5] >> (m_tile & 31) & 1u))) {
         constexpr int kGroups = kBlockM / kRowsPerReadyFlag;      // 16 flags per m-tile
@@ -452,7 +455,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const int kb0 = split * p.kb_per_split;
         const int kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
         // expert tiles: as many copies of a_box_rows rows as the tile's live rows take
-        const int a_rows = p.tile_rows ? (p.tile_rows[m_tile] + p.a_box_rows - 1) / p.a_box_rows * p.a_box_rows : p.a_box_rows;
+        const int a_rows = EXPERTS ? (p.tile_rows[m_tile] + p.a_box_rows - 1) / p.a_box_rows * p.a_box_rows : p.a_box_rows;
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, 0x100)) { ok = false; break; }
           uint8_t* sa = smem + stage * Cfg::kStageBytes;
@@ -464,7 +467,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             if (++sc_slot == kScaleSlots) sc_slot = 0;
           }
           tma_load_2d(sa, &tmap_a, &full[stage], kb * kElemsPerRow, m_tile * kBlockM);
-          if (p.tile_rows)
+          if (EXPERTS)
             for (int r = p.a_box_rows; r < a_rows; r += p.a_box_rows)
               tma_load_2d(sa + r * kRowBytes, &tmap_a, &full[stage], kb * kElemsPerRow, m_tile * kBlockM + r);
           if (p.epi_mode == 1) {
@@ -477,7 +480,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                           ((c & 1) ? p.act_cols : 0) + a0 + (c >> 1) * 32);
           } else {
             tma_load_2d(sa + Cfg::kABytes, &tmap_b, &full[stage], kb * kElemsPerRow,
-                        (p.tile_expert ? p.tile_expert[m_tile] * p.expert_n : 0) + n_tile * BLOCK_N);
+                        (EXPERTS ? p.tile_expert[m_tile] * p.expert_n : 0) + n_tile * BLOCK_N);
           }
           if (pf_on) pf_step();
           if (tl && item == (int)blockIdx.x && kb == kb0) tl[4] = clock64();
@@ -501,7 +504,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       uint32_t stage = 0, phase = 0, acc_iter = 0;
       bool ok = true;
       for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-        const int split = item_pos(p, item, m_tiles).split;
+        const int split = item_pos<EXPERTS>(p, item, m_tiles).split;
         const int kb0 = split * p.kb_per_split;
         const int kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
         if (!FP8) {
@@ -595,7 +598,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     // This loop never exits early: the split-K path below uses named barriers that need all eight warps.
     // Once a wait has failed (`ok` false) the remaining items only walk the barriers.
     for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
-      const ItemPos ip = item_pos(p, item, m_tiles);
+      const ItemPos ip = item_pos<EXPERTS>(p, item, m_tiles);
       const int m_tile = ip.m_tile;
       const int n_tile = ip.n_tile;
       const int split = ip.split;
@@ -615,7 +618,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           const int r = i / nkb, g = i - r * nkb;
           // SwiGLU mode: row 0 = the gate rows' block, row 1 = the up rows' block of this tile's activation columns
           const int nb = p.epi_mode == 1 ? ((r ? p.act_cols : 0) + n_tile * (BLOCK_N / 2)) / 128 : (n_tile * BLOCK_N) / 128 + r;
-          const float* bsrc = p.b_scale + (p.tile_expert ? (size_t)p.tile_expert[m_tile] * p.b_scale_expert_stride : 0);
+          const float* bsrc = p.b_scale + (EXPERTS ? (size_t)p.tile_expert[m_tile] * p.b_scale_expert_stride : 0);
           bs_buf[r * Cfg::kBScaleMax + g] = (nb * 128 < p.N) ? __ldg(bsrc + (size_t)nb * p.b_scale_ld + kb0 + g) : 0.f;
         }
         asm volatile("bar.sync 1, %0;\n" ::"n"(32 * kEpiWarps));
@@ -1022,7 +1025,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
         asm volatile("bar.sync 1, %0;\n" ::"n"(32 * kEpiWarps));
       } else
-      if (store_now && m < (p.tile_rows ? m_tile * kBlockM + p.tile_rows[m_tile] : M_rows)) {
+      if (store_now && m < (EXPERTS ? m_tile * kBlockM + p.tile_rows[m_tile] : M_rows)) {
         __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)m * p.ldc;
         if (!FP8 && p.bias != nullptr) {
 #pragma unroll
@@ -1260,18 +1263,18 @@ static int make_tmap_kmajor(CUtensorMap* out, const void* ptr, uint64_t rows, ui
   return make_tmap_2d(out, ptr, rows, cols, ld, box_rows, esize, 128u, true);
 }
 
-template <int BLOCK_N, bool FP8, bool FUSE_AR = false, int EPW = epi_warps(BLOCK_N, FP8)>
+template <int BLOCK_N, bool FP8, bool FUSE_AR = false, int EPW = epi_warps(BLOCK_N, FP8), bool EXPERTS = false>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t st) {
   using Cfg = GemmCfg<BLOCK_N>;
-  auto kern = gemm_tcgen05_kernel<BLOCK_N, FP8, FUSE_AR, EPW, false>;
+  auto kern = gemm_tcgen05_kernel<BLOCK_N, FP8, FUSE_AR, EPW, false, EXPERTS>;
   if constexpr (!FUSE_AR) {
-    if (p.timeline != nullptr) kern = gemm_tcgen05_kernel<BLOCK_N, FP8, FUSE_AR, EPW, true>;
+    if (p.timeline != nullptr) kern = gemm_tcgen05_kernel<BLOCK_N, FP8, FUSE_AR, EPW, true, EXPERTS>;
   }
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), Cfg::kSmemBytes) != cudaSuccess) return -20;
   if (p.cluster_splits > 1)
     return launch_chain_cluster(true, (unsigned)p.cluster_splits, kern, dim3(grid), dim3(gemm_threads_w(EPW, FUSE_AR)),
                                 (size_t)Cfg::kSmemBytes, st, ta, tb, p) == cudaSuccess ? 0 : -21;
-  return launch_chain_if(p.m_tiles <= 2 && p.tile_expert == nullptr, kern, dim3(grid), dim3(gemm_threads_w(EPW, FUSE_AR)),
+  return launch_chain_if(!EXPERTS && p.m_tiles <= 2, kern, dim3(grid), dim3(gemm_threads_w(EPW, FUSE_AR)),
                          (size_t)Cfg::kSmemBytes, st, ta, tb, p) == cudaSuccess ? 0 : -21;
 }
 
@@ -1520,13 +1523,13 @@ extern "C" int atlas_gemm_grouped(int kind, const void* A, const void* B, void* 
   int grid = (int)(items < num_sms ? items : num_sms);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (kind == 1) {
-    if (block_n == 64) return launch_gemm<64, true>(ta, tb, p, grid, st);
-    if (block_n == 128) return launch_gemm<128, true>(ta, tb, p, grid, st);
-    return launch_gemm<256, true>(ta, tb, p, grid, st);
+    if (block_n == 64) return launch_gemm<64, true, false, epi_warps(64, true), true>(ta, tb, p, grid, st);
+    if (block_n == 128) return launch_gemm<128, true, false, epi_warps(128, true), true>(ta, tb, p, grid, st);
+    return launch_gemm<256, true, false, epi_warps(256, true), true>(ta, tb, p, grid, st);
   }
-  if (block_n == 64) return launch_gemm<64, false>(ta, tb, p, grid, st);
-  if (block_n == 128) return launch_gemm<128, false>(ta, tb, p, grid, st);
-  return launch_gemm<256, false>(ta, tb, p, grid, st);
+  if (block_n == 64) return launch_gemm<64, false, false, epi_warps(64, false), true>(ta, tb, p, grid, st);
+  if (block_n == 128) return launch_gemm<128, false, false, epi_warps(128, false), true>(ta, tb, p, grid, st);
+  return launch_gemm<256, false, false, epi_warps(256, false), true>(ta, tb, p, grid, st);
 }
 
 // Row-parallel GEMM fused with its all-reduce.  Every rank calls this with its K-shard of A and B.
