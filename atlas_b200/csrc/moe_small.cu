@@ -15,7 +15,10 @@
 // same order.  Block scales multiply the f16 weights (exact), the per-row global scale the fp32 result.
 // Tiles of at most eight rows (most of a decode step's) stage their activations for the whole of K at once and then stream the weights
 // four spans ahead without a barrier; the others stage 256 k at a time.  Bound by the weight stream: 12 tokens x 8 of 128 experts,
-// 1536 x 2048 58.7 to 45 us; 2048 x 768 stays at 28 us.
+// 1536 x 2048 58.7 to 45 us; 2048 x 768 stays at 28 us.  The spans in flight take twice the registers (128 a thread), so that half as many
+// blocks fit on an SM: steps whose tiles are mostly fuller, or whose K is too long to stage, run the kernel without that path (FEW false, 64
+// registers).  The pair of products with and without it: 48 tokens x 4 of 32 experts (2048, 2048) 113 and 127 us, 100 tokens 178 and 162;
+// 200 x 8 of 128 (2048, 768) 256 and 209; 64 x 2 of 16 (5120, 8192) 631 and 520.
 // Reference ops replaced: moe_w4a16_grouped_gemv*.cu / w4a16_gemv*.cu (kernels/gb10/common).
 #include <cuda_fp4.h>
 #include <cuda_fp16.h>
@@ -96,7 +99,7 @@ ATLAS_DEVICE int small_place(int k) {
   return (k & ~127) + ((in_span & 31) >> 2) * 16 + (in_span >> 5) * 4;
 }
 
-template <int MODE>
+template <int MODE, bool FEW>
 __global__ void __launch_bounds__(kSmThreads)
 moe_small_w4_kernel(const SmallMoeParams p) {
   extern __shared__ __align__(16) __half xs[];
@@ -131,7 +134,7 @@ moe_small_w4_kernel(const SmallMoeParams p) {
   const uint8_t* s_lo = p.sc + wrow * (p.K >> 4) + 2 * t;
   const uint8_t* s_hi = s_lo + 8ll * (p.K >> 4);
   const float gs_lo = p.gs[wrow], gs_hi = p.gs[wrow + 8];
-  const bool few = n_live <= kSmFew && p.K <= kSmFewK;
+  const bool few = FEW && n_live <= kSmFew;
 
   for (int pass0 = 0; pass0 < n_live; pass0 += kSmTokens) {
     const int n_tok = min(kSmTokens, n_live - pass0);
@@ -248,9 +251,10 @@ using namespace atlas;
 // mode 1: x [T, K] token rows (gathered through row_token), out [max_rows, I] = silu(gate) * up, N = 2 I rows per expert
 // mode 0: x [max_rows, K] sorted rows, out [max_rows, N]
 // K % 256 == 0; mode 1: I % 32 == 0; mode 0: N % 64 == 0.  max_tiles bounds the grid; CTAs past *num_tiles return.
+// few: most tiles have at most eight rows.
 extern "C" int atlas_moe_small_w4(int mode, const void* x, long long ldx, const int* row_token, const int* tile_expert,
                                   const int* num_tiles, int max_tiles, const void* w, const void* sc, const float* gs,
-                                  void* out, long long ldo, int K, int N, void* stream) {
+                                  void* out, long long ldo, int K, int N, int few, void* stream) {
   if (max_tiles <= 0) return 0;
   if (K % kSmKc || (ldx % 4)) return -1;
   SmallMoeParams p;
@@ -261,11 +265,15 @@ extern "C" int atlas_moe_small_w4(int mode, const void* x, long long ldx, const 
   p.K = K; p.N = N; p.I = N / 2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (N % 64) return -2;
-  const int smem = max(kSmTokens * kSmRow, K <= kSmFewK ? kSmFew * (K + 16) : 0) * (int)sizeof(__half);
+  const bool whole = few && K <= kSmFewK;
+  const int smem = max(kSmTokens * kSmRow, whole ? kSmFew * (K + 16) : 0) * (int)sizeof(__half);
   auto launch = [&](auto kern, int blocks) {
-    if (smem > 16 * 1024 && ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) != cudaSuccess) return -20;
-    launch_chain(kern, dim3(blocks, max_tiles), dim3(kSmThreads), smem, st, p);
+    if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) != cudaSuccess) return -20;
+    // The down product starts the ordinary way: blocks of an early start fill the SMs that the first product leaves first, eight to one, and a
+    // small grid stays on those (2 tokens x 2 of 16 experts, 5120 x 8192: 55 us, early 100 to 190).
+    launch_chain_if(mode == 1, kern, dim3(blocks, max_tiles), dim3(kSmThreads), smem, st, p);
     return cudaGetLastError() == cudaSuccess ? 0 : -20;
   };
-  return mode == 1 ? launch(moe_small_w4_kernel<1>, p.I / 32) : launch(moe_small_w4_kernel<0>, N / 64);
+  if (mode == 1) return whole ? launch(moe_small_w4_kernel<1, true>, p.I / 32) : launch(moe_small_w4_kernel<1, false>, p.I / 32);
+  return whole ? launch(moe_small_w4_kernel<0, true>, N / 64) : launch(moe_small_w4_kernel<0, false>, N / 64);
 }

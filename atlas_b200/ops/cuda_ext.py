@@ -235,6 +235,7 @@ def _ones(n: int, dev) -> torch.Tensor:
 
 _SMALL_MOE = os.environ.get("ATLAS_MOE_SMALL", "1") not in ("0", "false")
 SMALL_MOE_ROWS_PER_EXPERT = 16
+SMALL_MOE_FEW_PER_EXPERT = 6            # rows per expert, on average, up to which most tiles have at most eight
 
 
 def _small_moe_ok(pairs: int, E: int, H: int, I: int) -> bool:
@@ -244,7 +245,7 @@ def _small_moe_ok(pairs: int, E: int, H: int, I: int) -> bool:
 def _bind_small(lib) -> None:
     if not getattr(lib, "_small_moe_bound", False):
         vp, i32, ll = C.c_void_p, C.c_int, C.c_longlong
-        lib.atlas_moe_small_w4.argtypes = [i32, vp, ll, vp, vp, vp, i32, vp, vp, vp, vp, ll, i32, i32, vp]
+        lib.atlas_moe_small_w4.argtypes = [i32, vp, ll, vp, vp, vp, i32, vp, vp, vp, vp, ll, i32, i32, i32, vp]
         lib._small_moe_bound = True
 
 
@@ -337,14 +338,15 @@ def _moe_local(x, topk_w, topk_ids, experts, e_lo, addend: Optional[torch.Tensor
         # decode-size batch on NVFP4 experts: a few rows per expert, so stream the weights through the register-level
         # dequant kernel (rows gathered by token inside it, SiLU fused) instead of 128-row tcgen05 tiles
         _bind_small(lib)
+        few = int(T * k <= SMALL_MOE_FEW_PER_EXPERT * E)
         act = torch.empty(max_rows, I, dtype=torch.bfloat16, device=dev)
         K._check(lib.atlas_moe_small_w4(1, x.data_ptr(), x.stride(0), row_token.data_ptr(), tile_expert.data_ptr(),
                                         num_tiles.data_ptr(), max_rows // 128, w13.data_ptr(), s13[0].data_ptr(),
-                                        s13[1].data_ptr(), act.data_ptr(), I, H, 2 * I, st), "moe_small_gate_up")
+                                        s13[1].data_ptr(), act.data_ptr(), I, H, 2 * I, few, st), "moe_small_gate_up")
         y = torch.empty(max_rows, H, dtype=torch.bfloat16, device=dev)
         K._check(lib.atlas_moe_small_w4(0, act.data_ptr(), I, row_token.data_ptr(), tile_expert.data_ptr(),
                                         num_tiles.data_ptr(), max_rows // 128, w2.data_ptr(), s2[0].data_ptr(),
-                                        s2[1].data_ptr(), y.data_ptr(), H, I, H, st), "moe_small_down")
+                                        s2[1].data_ptr(), y.data_ptr(), H, I, H, few, st), "moe_small_down")
         return _finish(lib, y, slot_of, topk_w, T, k, H, addend, fused_comm, grouped, dev, st)
     if kind == 1:
         xq = torch.empty(max_rows, H, dtype=FP8, device=dev)

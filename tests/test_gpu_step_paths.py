@@ -257,6 +257,65 @@ def test_delta_net_decode_graph_equals_eager_steps(K, n):
             v.copy_(torch.zeros(v.shape, device=DEV).to(v.dtype))
         got = []
         for s in range(3):
+@pytest.mark.parametrize("counts", [[1, 0, 8], [9, 7, 33, 2], [70, 3]])
+@pytest.mark.parametrize("H,I", [(256, 256), (4096, 256), (4352, 512)])
+def test_small_nvfp4_experts_with_and_without_whole_rows_staged(K, counts, H, I):
+    """Tiles around eight rows and more than one pass of 32, K at and behind the longest that is staged whole: both kernels give the same
+    bits (the same MMAs in the same order), and 64 bits up to the rounding of intermediate rows and results to bf16 (2^-9 each, the
+    first through a product)."""
+    from atlas_b200.ops import cuda_ext
+    lib = K.lib()
+    cuda_ext.bind(lib)
+    cuda_ext._bind_small(lib)
+    g = torch.Generator(device=DEV).manual_seed(sum(counts) + H)
+    E, T = len(counts), sum(counts)
+    ids = torch.cat([torch.full((n,), e) for e, n in enumerate(counts)]).int().to(DEV).view(-1, 1)
+    tiles = T // 128 + min(T, E)
+    slot, rows = torch.empty(T, dtype=torch.int32, device=DEV), torch.empty(tiles * 128, dtype=torch.int32, device=DEV)
+    te, tr, nt = (torch.zeros(m, dtype=torch.int32, device=DEV) for m in (tiles, tiles, 2))
+    K._check(lib.atlas_moe_align(ids.data_ptr(), T, 1, 0, E, slot.data_ptr(), rows.data_ptr(), te.data_ptr(), tr.data_ptr(), None, nt.data_ptr(), tiles * 128,
+                                 K._status_ptr[K._dev(ids)], K._stream()), "moe_align")
+    w13, w2 = _nvfp4(g, E, 2 * I, H), _nvfp4(g, E, H, I)
+    x = (torch.randn(T, H, generator=g, device=DEV) * 0.1).bfloat16()
+    got = []
+    for few in (0, 1):
+        act, y = (torch.zeros(tiles * 128, n, dtype=torch.bfloat16, device=DEV) for n in (I, H))
+        K._check(lib.atlas_moe_small_w4(1, x.data_ptr(), H, rows.data_ptr(), te.data_ptr(), nt.data_ptr(), tiles, w13[0].data_ptr(), w13[1].data_ptr(),
+                                        w13[2].data_ptr(), act.data_ptr(), I, H, 2 * I, few, K._stream()), "up")
+        K._check(lib.atlas_moe_small_w4(0, act.data_ptr(), I, rows.data_ptr(), te.data_ptr(), nt.data_ptr(), tiles, w2[0].data_ptr(), w2[1].data_ptr(),
+                                        w2[2].data_ptr(), y.data_ptr(), H, I, H, few, K._stream()), "down")
+        got.append((act[slot.long()], y[slot.long()]))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    for e in range(E):
+        r = (ids[:, 0] == e)
+        if int(r.sum()):
+            gate, up = (x[r].double() @ _nvfp4_value(w13, e, 2 * I).t()).bfloat16().double().chunk(2, -1)
+            want = (torch.nn.functional.silu(gate) * up).bfloat16().double() @ _nvfp4_value(w2, e, H).t()
+            assert _rel(got[1][1][r], want) < 2 ** -8
+
+
+@pytest.mark.parametrize("C,ld,off", [(8, 8, 0), (12, 12, 0), (2052, 4104, 4), (1024, 1028, 4), (40, 44, 0), (1023, 1023, 0)])
+@pytest.mark.parametrize("taps,rows,silu", [(4, 261, 1), (2, 300, 2), (3, 1031, 1), (1, 257, 0), (4, 6200, 1)])
+def test_convolution_of_rows_at_any_alignment(K, C, ld, off, taps, rows, silu):
+    """bf16 rows that start on 16, 8 or 2 bytes, two sequences, more and fewer rows than the widest loads are taken for: against 64 bits
+    (fp32 sums, a result rounded to bf16)."""
+    from atlas_b200.ops import cuda_gdn, cuda_recurrent
+    g = torch.Generator(device=DEV).manual_seed(C + rows)
+    x = torch.randn(rows, ld + off, generator=g, device=DEV).bfloat16()[:, off:off + C]
+    w = (torch.randn(C, taps, generator=g, device=DEV) * 0.5).bfloat16()
+    bias = torch.randn(C, generator=g, device=DEV).bfloat16()
+    state = torch.randn(2, C, max(1, taps - 1), generator=g, device=DEV).bfloat16()[:, :, :taps - 1].contiguous()
+    lens = [rows - 5, 5]
+    meta = cuda_gdn._Meta(lens, [1, 0], [True, False], DEV)
+    y = torch.zeros(rows, C, dtype=torch.bfloat16, device=DEV)
+    cuda_recurrent.conv_silu(x, w, bias, state, meta, y, False, silu=silu)
+    for (lo, hi), win in (((0, rows - 5), state[1]), ((rows - 5, rows), torch.zeros_like(state[0]))):
+        full = torch.cat([win.double().t(), x[lo:hi].double()])
+        want = (full.unfold(0, taps, 1) * w.double()).sum(-1) + bias.double()
+        want = torch.nn.functional.silu(want) if silu else want
+        assert float(((y[lo:hi].double() - want).abs() / (want.abs() + 1e-2)).max()) < 2 ** -8
+
+
             b = ForwardBatch.build([[7 * i + s + 1] for i in range(n)], [4 + s] * n, [[2 * i, 2 * i + 1] for i in range(n)], 16, device=DEV,
                                    state_slots=list(range(n)), has_state=[True] * n)
             with torch.inference_mode():
