@@ -6,6 +6,8 @@
 //
 // Activations are bf16 or fp32 (template parameter T).
 // Reference op replaced: kernels/gb10/common/causal_conv1d.cu.
+#include <type_traits>
+
 #include "common.cuh"
 #include "host_api.h"
 #include "vec_io.cuh"
@@ -236,12 +238,20 @@ static int launch_conv(const void* x, long long ldx, const void* w, const void* 
   T* yp = reinterpret_cast<T*>(y);
   const int span = rows <= 256 ? 1 : kConvRows;
   const unsigned gx = (rows + span - 1) / span;
-  // 16 bytes of a row per thread: 8 bf16 channels or 4 fp32 ones
+  // 16 bytes of a row per thread: 8 bf16 channels or 4 fp32 ones.  Rows of bf16 that start on 8 bytes only (C or the stride 4 mod 8) take
+  // 4 channels (8192 rows of 4100: 125 us with a channel per thread, 45 us so), and so do steps that leave most threads of the chip idle
+  // otherwise (300 rows of 10240: 9.2 us with 4, 11.7 with 8; 4000 of 2048, two taps: 10.4, 12.5; 1500 of 10240: 23.6, 21.7).
   constexpr int V = 16 / sizeof(T);
-  if (kTaps > 0 && rows > 256 && C % V == 0 && vec_ok<T, V>(x, ldx) && vec_ok<T, V>(y, ldy) && vec_ok<T, V>(w, 0))
-    launch_chain_if(false, conv1d_kernel<T, kTaps, (kTaps > 0 ? V : 1)>, dim3(gx, (C / V + 127) / 128), dim3(128), 0, st, xp, ldx, wp, bp, C, W,
+  const bool large = V == 4 || (long long)rows * C >= (12ll << 20);
+  auto wide = [&](auto vec) {
+    constexpr int N = decltype(vec)::value;
+    if (kTaps == 0 || rows <= 256 || C % N || !vec_ok<T, N>(x, ldx) || !vec_ok<T, N>(y, ldy) || !vec_ok<T, V>(w, 0)) return false;
+    constexpr int threads = kTaps < 4 ? 256 : 128;            // (4000 rows of 2048 bf16, two taps: 10.4 us, with 128 11.5)
+    launch_chain_if(false, conv1d_kernel<T, kTaps, (kTaps > 0 ? N : 1)>, dim3(gx, (C / N + threads - 1) / threads), dim3(threads), 0, st, xp, ldx, wp, bp, C, W,
                     sp, seq, qsl, slots, has, yp, ldy, rows, after, advance, span);
-  else
+    return true;
+  };
+  if (!(large && wide(std::integral_constant<int, V>())) && (V == 4 || !wide(std::integral_constant<int, 4>())))
     launch_chain_if(rows <= 256, conv1d_kernel<T, kTaps, 1>, dim3(gx, (C + 255) / 256), dim3(256), 0, st, xp, ldx, wp, bp, C, W, sp, seq, qsl,
                     slots, has, yp, ldy, rows, after, advance, span);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
