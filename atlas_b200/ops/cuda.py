@@ -296,9 +296,11 @@ def gemm_plan(M: int, N: int, K: int, kind: int, sms: int) -> Tuple[int, int]:
         bn = 256          # fp8: half the per-k-group buffer handshakes per FLOP and 0.75x the shared-memory fill of 128
     elif m_tiles * ((N + 127) // 128) >= sms:
         bn = 128
-    elif m_tiles == 1 and K >= 8192 and N % 128 == 0:
-        # decode rows, long K: fewer, wider tiles and more K splits (FP8 128 x 4096 x 14336: 35.5 -> 31.1 us; bf16 32 x 4096 x 21504:
-        # 56.3 -> 38.2 us, x 8192: 25.6 -> 19.8 us)
+    elif m_tiles == 1 and K >= 8192 and N % 128 == 0 and (kind == 1 or sms // (N // 128) <= 4):
+        # decode rows, long K: fewer, wider tiles and more K splits (FP8 128 x 4096 x 14336: 35.5 -> 31.1 us; bf16 1 to 128 rows, K 8192 to
+        # 21504, cold: N 4096 30.7 to 61 -> 28 to 51, 5120 45 to 102 -> 33 to 63, 9216 49 to 107 -> 44 to 90).  bf16 up to four splits, which
+        # meet in a cluster: narrower outputs get more splits than 64-wide tiles need (N 512 20 -> 33, 1024 19 -> 29, 2048 22.5 -> 26,
+        # 3072 x 8192 25 -> 29)
         bn = 128
     elif m_tiles == 1 and (N + 63) // 64 > sms:
         # decode rows: one wave of 128-wide tiles (up to sms: the rule above) where 64-wide ones would leave a second wave nearly empty

@@ -1,0 +1,15 @@
+"""Rules that choose a kernel or a tile by sizes, at the sizes where they turn.  The times beside them were measured on a B200."""
+import pytest
+
+from atlas_b200.ops import cuda as K
+
+SMS = 148
+
+
+@pytest.mark.parametrize("M,N,Kd,want", [
+    (1, 4096, 8192, (128, 4)), (128, 4096, 21504, (128, 4)), (32, 5120, 14336, (128, 3)), (8, 9216, 8192, (128, 2)),      # meet in a cluster
+    (1, 512, 8192, (64, 16)), (32, 1024, 14336, (64, 9)), (128, 2048, 8192, (64, 4)), (8, 3072, 8192, (64, 3)),          # narrow: 64-wide tiles
+    (32, 4096, 8191, (64, 2)), (129, 4096, 8192, (64, 1)),
+])
+def test_bf16_decode_products_of_long_k(M, N, Kd, want):
+    assert K.gemm_plan(M, N, Kd, 0, SMS) == want
