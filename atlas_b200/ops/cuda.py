@@ -284,6 +284,17 @@ _FORCE_BLOCK_N = int(os.environ.get("ATLAS_GEMM_BLOCK_N", "0"))
 _FORCE_SPLITS = int(os.environ.get("ATLAS_GEMM_SPLITS", "0"))
 
 
+def _wide_cut_pays(m_tiles: int, N: int, K: int, sms: int) -> bool:
+    """FP8 rows on 256-wide tiles whose last one is cut off (N no multiple of 256).  A wide tile costs 2.35 narrow ones at K = 1024, 2 at
+    2048, 1.8 at 3072 and 1.7 at 4096 (it has more to set up and less to overlap it with), and its last wave is twice as coarse: 1024 rows of
+    4992 x 4096 are three narrow waves, 54 us, or two wide ones, 58 us; 4500 x 12352 at K 1024 135 and 158 us, at 2048 221 and 214,
+    at 4096 378 and 322."""
+    if K < 2048:
+        return False
+    wide, narrow = (-(-m_tiles * ((N + w - 1) // w) // sms) for w in (256, 128))
+    return 2 * wide <= narrow * min(1.2, 1.0 + (K - 2048) / 8192)
+
+
 def gemm_plan(M: int, N: int, K: int, kind: int, sms: int) -> Tuple[int, int]:
     """(block_n, k-splits) for a problem: fill the SMs first with tiles, then with K splits."""
     k_blocks = (K + (128 if kind == 1 else 64) - 1) // (128 if kind == 1 else 64)
@@ -292,7 +303,7 @@ def gemm_plan(M: int, N: int, K: int, kind: int, sms: int) -> Tuple[int, int]:
         bn = _FORCE_BLOCK_N
     elif kind == 0 and m_tiles * ((N + 255) // 256) >= 2 * sms and -N % 256 * 16 <= N:
         bn = 256          # bf16 accumulates in TMEM across K; a last tile that is cut off costs at most 1/16
-    elif kind == 1 and m_tiles * ((N + 255) // 256) >= sms and -N % 256 * 16 <= N:
+    elif kind == 1 and m_tiles * ((N + 255) // 256) >= sms and (N % 256 == 0 or _wide_cut_pays(m_tiles, N, K, sms)):
         bn = 256          # fp8: half the per-k-group buffer handshakes per FLOP and 0.75x the shared-memory fill of 128
     elif m_tiles * ((N + 127) // 128) >= sms:
         bn = 128

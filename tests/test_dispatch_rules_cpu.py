@@ -13,3 +13,15 @@ SMS = 148
 ])
 def test_bf16_decode_products_of_long_k(M, N, Kd, want):
     assert K.gemm_plan(M, N, Kd, 0, SMS) == want
+
+
+@pytest.mark.parametrize("M,N,Kd,want", [
+    (4500, 12352, 1024, 128), (8192, 18560, 1536, 128),                     # a wide tile of short K costs more than two narrow ones
+    (4500, 12352, 2048, 256), (8192, 12352, 2048, 128), (8192, 12352, 4096, 256), (2500, 4992, 2048, 256),
+    (1024, 4992, 4096, 128), (300, 18560, 4096, 128), (1024, 6272, 8192, 128),     # two wide waves for three narrow ones
+    (1024, 12352, 4096, 256), (517, 12352, 3072, 256),
+    (4500, 12288, 1024, 256), (1024, 4864, 1024, 256),                      # whole tiles: as ever
+    (500, 4992, 4096, 128),                                                  # fewer wide tiles than SMs
+])
+def test_fp8_products_whose_last_wide_tile_is_cut_off(M, N, Kd, want):
+    assert K.gemm_plan(M, N, Kd, 1, SMS)[0] == want
