@@ -705,7 +705,8 @@ def paged_attention(q, k_cache, v_cache, batch, scale, k_scale, v_scale, sliding
                                        batch.query_start_loc.data_ptr(), 0, nd, float(scale), float(k_scale),
                                        float(v_scale), Hq, Hkv, D, bs, window, splits, _ptr(po), _ptr(pml), _status_ptr[d], st),
                "attn_decode")
-    if batch.num_seqs > nd and _tc_prefill_ok(q, Hq, Hkv, D, bs, window, k_cache):
+    if (batch.num_seqs > nd and _tc_prefill_ok(q, Hq, Hkv, D, bs, window, k_cache)
+            and not _short_prompts_fill_waves(batch, nd, Hq, Hkv, D, _num_sms[d], 16)):
         # tensor-core (tcgen05) chunk attention: tiles of 128 / G query tokens, all G heads of a kv head per tile
         tdev, n_tiles, _ = _tc_tiles(q, batch, nd, 128 // (Hq // Hkv))
         rc = lib().atlas_attn_prefill_tc(q.data_ptr(), q.stride(0), out.data_ptr(), Hq * D, k_cache.data_ptr(),
@@ -849,7 +850,8 @@ def _paged_attention_kv16(q, out, k_cache, v_cache, batch, scale, window, d, sca
                                             bt.data_ptr(), bt.stride(0), batch.seq_lens.data_ptr(), batch.query_start_loc.data_ptr(),
                                             0, nd, float(scale), Hq, Hkv, D, bs, window, splits, _ptr(po), _ptr(pml), st, chunk,
                                             _ptr(sinks), softcap, *bias), "attn_decode_kv16")
-    if batch.num_seqs > nd and not fp4 and _TC_PREFILL and bs == 16 and (D <= 128 or D == 256) and Hq // Hkv <= 128:
+    if (batch.num_seqs > nd and not fp4 and _TC_PREFILL and bs == 16 and (D <= 128 or D == 256) and Hq // Hkv <= 128
+            and not _short_prompts_fill_waves(batch, nd, Hq, Hkv, D, _num_sms[d], 8)):
         # tcgen05 tiles of 128 // G query tokens; 1 = a shape the kernel does not take
         tdev, n_tiles, _ = _tc_tiles(q, batch, nd, 128 // (Hq // Hkv))
         if not getattr(L, "_tc16_bound", False):
@@ -922,6 +924,15 @@ def _bf16_cached(t: torch.Tensor) -> torch.Tensor:
 
 
 _TC_PREFILL = os.environ.get("ATLAS_ATTN_TC", "1") not in ("0", "false")
+
+
+def _short_prompts_fill_waves(batch, nd: int, Hq: int, Hkv: int, D: int, sms: int, most: int) -> bool:
+    """Many prompts of a few tokens, nothing cached, on 256-wide heads: a tcgen05 tile costs some 12 us whatever it holds, so more tiles than
+    SMs cost more than the general kernel's rows while no row sees more than ``most`` keys (FP8 32 prompts of 2 to 16 tokens on 8 kv heads: 13
+    to 19 and 21 to 23 us, of 40: 50 and 41; bf16 on 16 kv heads, 5 tokens: 29 and 46 us, 16: 34 and 34)."""
+    tok = 128 // (Hq // Hkv)
+    return (D == 256 and max(batch.seq_lens_host[nd:]) <= most
+            and sum(-(-n // tok) for n in batch.query_lens_host[nd:]) * Hkv > sms)
 
 
 def _tc_prefill_ok(q, Hq, Hkv, D, bs, window, k_cache) -> bool:

@@ -1,4 +1,6 @@
 """Rules that choose a kernel or a tile by sizes, at the sizes where they turn.  The times beside them were measured on a B200."""
+import types
+
 import pytest
 
 from atlas_b200.ops import cuda as K
@@ -25,3 +27,13 @@ def test_bf16_decode_products_of_long_k(M, N, Kd, want):
 ])
 def test_fp8_products_whose_last_wide_tile_is_cut_off(M, N, Kd, want):
     assert K.gemm_plan(M, N, Kd, 1, SMS)[0] == want
+
+
+@pytest.mark.parametrize("ctx,q,seqs,Hq,Hkv,D,most,want", [
+    (0, 5, 32, 32, 8, 256, 16, True), (0, 16, 32, 32, 8, 256, 16, True), (0, 17, 32, 32, 8, 256, 16, False),
+    (500, 5, 32, 32, 8, 256, 16, False), (0, 5, 32, 16, 2, 256, 16, False), (0, 5, 32, 32, 8, 128, 16, False),
+    (0, 5, 32, 32, 16, 256, 8, True), (0, 9, 32, 32, 16, 256, 8, False),
+])
+def test_many_short_prompts_on_wide_heads(ctx, q, seqs, Hq, Hkv, D, most, want):
+    batch = types.SimpleNamespace(seq_lens_host=[9000] + [ctx + q] * seqs, query_lens_host=[1] + [q] * seqs)        # one decode row in front
+    assert K._short_prompts_fill_waves(batch, 1, Hq, Hkv, D, SMS, most) is want
