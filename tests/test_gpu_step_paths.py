@@ -238,25 +238,6 @@ def test_plain_nvfp4_product_of_two_row_tiles(K, M, N, Kd, sms):
     assert _rel(got[0][:M], x.double() @ _nvfp4_value(w, 0, N).t()) < 2 ** -9 + 1e-5
 
 
-# ----------------------------------------------------------------------------- decode graphs of Gated DeltaNet models
-@pytest.mark.parametrize("n", [1, 3, 9])
-def test_delta_net_decode_graph_equals_eager_steps(K, n):
-    """Three decode steps from the same states, replayed and eager (padding rows included): the same bits."""
-    cfg = PRESETS["tiny-hybrid"]("bfloat16")
-    model = build_model(cfg, device=DEV, with_mtp=False).init_random(0, max_pos=256)
-    outs = []
-    for graphs in (True, False):
-        eng = LLMEngine(model, EngineConfig(max_seq_len=256, num_kv_blocks=64, max_num_seqs=n, max_batch_size=n, use_cuda_graphs=graphs,
-                                            enable_prefix_caching=False))
-        gen = torch.Generator(device=DEV).manual_seed(5)
-        for i, st in eng.cache.states.items():
-            st["h"][:n] = torch.randn(st["h"][:n].shape, generator=gen, device=DEV) * 0.1
-            st["conv"][:n] = torch.randn(st["conv"][:n].shape, generator=gen, device=DEV).bfloat16()
-        for k, v in eng.cache.kv.values():
-            k.copy_(torch.zeros(k.shape, device=DEV).to(k.dtype))
-            v.copy_(torch.zeros(v.shape, device=DEV).to(v.dtype))
-        got = []
-        for s in range(3):
 @pytest.mark.parametrize("counts", [[1, 0, 8], [9, 7, 33, 2], [70, 3]])
 @pytest.mark.parametrize("H,I", [(256, 256), (4096, 256), (4352, 512)])
 def test_small_nvfp4_experts_with_and_without_whole_rows_staged(K, counts, H, I):
@@ -316,6 +297,25 @@ def test_convolution_of_rows_at_any_alignment(K, C, ld, off, taps, rows, silu):
         assert float(((y[lo:hi].double() - want).abs() / (want.abs() + 1e-2)).max()) < 2 ** -8
 
 
+# ----------------------------------------------------------------------------- decode graphs of Gated DeltaNet models
+@pytest.mark.parametrize("n", [1, 3, 9])
+def test_delta_net_decode_graph_equals_eager_steps(K, n):
+    """Three decode steps from the same states, replayed and eager (padding rows included): the same bits."""
+    cfg = PRESETS["tiny-hybrid"]("bfloat16")
+    model = build_model(cfg, device=DEV, with_mtp=False).init_random(0, max_pos=256)
+    outs = []
+    for graphs in (True, False):
+        eng = LLMEngine(model, EngineConfig(max_seq_len=256, num_kv_blocks=64, max_num_seqs=n, max_batch_size=n, use_cuda_graphs=graphs,
+                                            enable_prefix_caching=False))
+        gen = torch.Generator(device=DEV).manual_seed(5)
+        for i, st in eng.cache.states.items():
+            st["h"][:n] = torch.randn(st["h"][:n].shape, generator=gen, device=DEV) * 0.1
+            st["conv"][:n] = torch.randn(st["conv"][:n].shape, generator=gen, device=DEV).bfloat16()
+        for k, v in eng.cache.kv.values():
+            k.copy_(torch.zeros(k.shape, device=DEV).to(k.dtype))
+            v.copy_(torch.zeros(v.shape, device=DEV).to(v.dtype))
+        got = []
+        for s in range(3):
             b = ForwardBatch.build([[7 * i + s + 1] for i in range(n)], [4 + s] * n, [[2 * i, 2 * i + 1] for i in range(n)], 16, device=DEV,
                                    state_slots=list(range(n)), has_state=[True] * n)
             with torch.inference_mode():
