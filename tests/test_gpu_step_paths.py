@@ -71,6 +71,25 @@ def test_expert_products_touch_live_rows_only(K, T, E, hot):
     assert _rel(got, want) < 0.02 if float(want.abs().max()) > 0 else float(got.abs().max()) == 0
 
 
+@pytest.mark.parametrize("T,E,H,I", [(30, 4, 256, 128), (60, 4, 256, 128), (300, 3, 4096, 2112)])
+def test_bf16_expert_products_by_copy_size_and_order(K, T, E, H, I):
+    """Rows copied 32, 64 and 128 at a time (15, 30 and 200 rows an expert), and experts of 34 MB (row tiles first): against an oracle that rounds
+    where the kernels do; what is left is the last rounding to bf16 and the few values before it that another order of the sums turns."""
+    torch.manual_seed(T + H)
+    ex = ExpertWeights.from_dense((torch.randn(E, 2 * I, H, device=DEV) * 0.02).bfloat16(), (torch.randn(E, H, I, device=DEV) * 0.02).bfloat16(), "dense")
+    w, ids = ref.moe_route(torch.randn(T, E, device=DEV), 2, True)
+    x = torch.randn(T, H, device=DEV).bfloat16()
+    got = K.moe_forward(x, w.contiguous(), ids.contiguous(), ex, 0, None, "auto")
+    assert K.check_status() == 0
+    want = torch.zeros(T, H, device=DEV)
+    for e in range(E):
+        t, j = (ids == e).nonzero(as_tuple=True)
+        g, u = (x[t].double() @ ex.w13[e].double().t()).bfloat16().float().chunk(2, -1)
+        o = (torch.nn.functional.silu(g) * u).bfloat16().double() @ ex.w2[e].double().t()
+        want.index_add_(0, t, o.bfloat16().float() * w[t, j].float()[:, None])
+    assert _rel(got, want) < 2 ** -8
+
+
 @pytest.mark.parametrize("T,k", [(75, 4), (1023, 4), (1024, 4), (2731, 3)])
 def test_expert_row_lists(K, T, k):
     """align: every routed pair has a row of its own inside its expert's segment, and the tiles say how many rows live (one CTA; a
