@@ -128,6 +128,7 @@ struct GemmParams {
   unsigned long long* timeline;
   const int* tile_expert;       // nullptr = plain GEMM (EXPERTS kernels only)
   const int* tile_rows;         // live rows of every tile, its leading ones: the others are neither copied nor stored
+  int rows_first;               // EXPERTS: order of the work items, see item_pos
   const int* num_m_tiles_ptr;   // device-side tile count (the host cannot know it)
   int expert_n;                 // output features per expert
   long long b_scale_expert_stride;
@@ -189,8 +190,11 @@ ATLAS_DEVICE ItemPos item_pos(const GemmParams& p, int item, int m_tiles) {
   ItemPos r;
   if (EXPERTS) {
     // Experts: the column tiles of a row tile one after the other, so that its rows come from HBM once and from L2 after that (row tiles
-    // first read 230 MB of rows again for every column tile: 8192 tokens x 10 of 512 experts, 878 and 844 us a layer).
-    r.m_tile = item / p.n_tiles; r.n_tile = item % p.n_tiles; r.split = 0;
+    // first read 230 MB of rows again for every column tile: 8192 tokens x 10 of 512 experts, 878 and 844 us a layer).  Weights of which one
+    // expert alone is a good part of L2 come from HBM for every row tile that way: row tiles first there (see rows_first).
+    if (p.rows_first) { r.m_tile = item % m_tiles; r.n_tile = item / m_tiles; }
+    else              { r.m_tile = item / p.n_tiles; r.n_tile = item % p.n_tiles; }
+    r.split = 0;
   } else if (p.cluster_splits > 1) {
     r.m_tile = 0; r.n_tile = item / p.cluster_splits; r.split = item % p.cluster_splits;
   } else {
@@ -1504,6 +1508,9 @@ extern "C" int atlas_gemm_grouped(int kind, const void* A, const void* B, void* 
   GemmParams p = {};
   p.timeline = g_gemm_timeline;
   p.a_box_rows = a_box; p.tile_rows = tile_rows;
+  // 8 experts of 28672 x 4096 and 4096 x 14336, bf16, 250 rows each: 1090 us with columns first, 958 with rows first (FP8 758 and 745); of
+  // 8 MB an expert (32 of 2048 x 2048, 1024 rows each) 633 and 723 us
+  p.rows_first = (long long)N * K * esize > (32ll << 20) ? 1 : 0;
   p.C = C; p.a_scale = a_scale; p.b_scale = b_scale; p.workspace = nullptr; p.counters = nullptr;
   p.status = status; p.ldc = ldc; p.sa_k = sa_k; p.M = max_rows; p.N = N; p.K = K;
   p.k_blocks = (K + elems_per_row - 1) / elems_per_row;
