@@ -170,8 +170,18 @@ def scratch(name: str, nbytes: int, device, zero_new=None) -> torch.Tensor:
 _scratch_alloc = None      # tests replace the allocator to exercise the policy without a GPU
 
 
+_scratch_retired: list = []      # buffers that graphs captured before a larger one was reserved
+
+
 def reserve_scratch(name: str, nbytes: int, device) -> torch.Tensor:
-    """Make sure ``name`` holds at least ``nbytes`` (call before any graph capture)."""
+    """Make sure ``name`` holds at least ``nbytes`` (call before any graph capture of the model that needs them).  Another model of the
+    process may have captured graphs by then: they keep the buffer they were captured with, and the larger one, at least twice its
+    size, serves everything after that."""
+    key = (device.index if device.index is not None else (torch.cuda.current_device() if device.type == "cuda" else -1), name)
+    buf = _scratch.get(key)
+    if _scratch_frozen and buf is not None and buf.numel() < nbytes:
+        _scratch_retired.append(_scratch.pop(key))
+        nbytes = max(nbytes, 2 * buf.numel())
     return scratch(name, nbytes, device)
 
 

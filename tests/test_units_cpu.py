@@ -578,6 +578,28 @@ def test_attention_scratch_is_reserved_once_and_never_replaced(preset, tp, monke
         K.scratch("attn_part_o", max(po, 1 << 20) + 1, dev)
 
 
+def test_a_later_model_may_reserve_more_scratch_than_captured_graphs_use(monkeypatch):
+    """An engine that is made after another one has captured its graphs, and needs larger partials: it gets them, the graphs keep theirs,
+    and a step that was not reserved for still raises."""
+    import gc
+    import weakref
+    from atlas_b200.ops import cuda as K
+    monkeypatch.setattr(K, "_scratch_alloc", lambda n, dev: torch.zeros(n, dtype=torch.uint8))
+    monkeypatch.setattr(K, "_scratch", {})
+    monkeypatch.setattr(K, "_scratch_retired", [])
+    monkeypatch.setattr(K, "_scratch_frozen", False)
+    dev = torch.device("cpu")
+    first = weakref.ref(K.reserve_scratch("attn_part_o", 2 << 20, dev))
+    K.freeze_scratch()
+    assert K.reserve_scratch("attn_part_o", 2 << 20, dev) is first()
+    second = K.reserve_scratch("attn_part_o", 3 << 20, dev)
+    gc.collect()
+    assert second.numel() == 4 << 20 and first() is not None and first().data_ptr() != second.data_ptr()
+    assert K.scratch("attn_part_o", 4 << 20, dev) is second
+    with pytest.raises(K.KernelError):
+        K.scratch("attn_part_o", (4 << 20) + 1, dev)
+
+
 def test_router_variants_reference():
     """Selection bias, group-limited routing, sqrt-softplus scores, static hash selection and the weight scale, each
     against a direct restatement of the published routing rule."""
