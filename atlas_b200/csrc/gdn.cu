@@ -610,24 +610,28 @@ extern "C" int atlas_gdn_recurrent(const void* y, long long ldy, const void* a, 
 // Chunked (64-token) evaluation of the same recurrence for prefill-sized steps of T rows: Dk = Dv = 128, whole sequences (no row
 // limit); a snapshot row inside a chunk simply ends that chunk early.  Sequences of fewer than row_lo rows are left out (a chunk costs
 // the same however few rows it has).  Same state layout and arguments as atlas_gdn_recurrent.
-// `work`: atlas_gdn_chunked_bytes(...) bytes, 16-byte aligned.  Returns 1 for shapes that only the recurrence takes.
+// `work`: atlas_gdn_chunked_bytes_within(limit, ...) bytes, 16-byte aligned.  Returns 1 for shapes that only the recurrence takes.
 static long long gdn_items(int T, int B, int snaps) { return T / kGC + (long long)B * (1 + snaps); }
 
-// Bytes of workspace for `heads` value heads at once (whole key heads); *heads: all of them while that stays within 256 MB (11 k rows of 32
-// heads and 16 key heads), else as many as do, in several pairs of launches.
-extern "C" long long atlas_gdn_chunked_bytes(int T, int B, int snaps, int Hk, int Hv, int* heads) {
+// Bytes of workspace for `heads` value heads at once (whole key heads); *heads: all of them while that stays within `limit` bytes, else as
+// many as do, but at least one key head's, in several pairs of launches.
+constexpr long long kGLimit = 256ll << 20;            // 11 k rows of 32 heads and 16 key heads
+extern "C" long long atlas_gdn_chunked_bytes_within(long long limit, int T, int B, int snaps, int Hk, int Hv, int* heads) {
   const int rep = Hv / Hk;
   const long long per_key_head = gdn_items(T, B, snaps) * ((kGMats + kGFactors) * 4ll * rep + kGRows * 2ll);
-  const long long n = max(1ll, min((long long)Hk, (256ll << 20) / max(per_key_head, 1ll)));
+  const long long n = max(1ll, min((long long)Hk, limit / max(per_key_head, 1ll)));
   *heads = (int)n * rep;
   return per_key_head * n;
 }
+extern "C" long long atlas_gdn_chunked_bytes(int T, int B, int snaps, int Hk, int Hv, int* heads) {
+  return atlas_gdn_chunked_bytes_within(kGLimit, T, B, snaps, Hk, Hv, heads);
+}
 
-extern "C" int atlas_gdn_chunked(const void* y, long long ldy, const void* a, long long lda, const void* b, long long ldb,
-                                 const float* A_log, const float* dt_bias, float* h, void* out, long long ldo,
-                                 const int* query_start_loc, const int* state_slots, const unsigned char* has_state,
-                                 const int* snap_rows, const int* snap_slots, int num_snaps_per_seq, int T, int B, int Hk, int Hv,
-                                 int Dk, int Dv, int commit, int row_lo, void* work, void* stream) {
+extern "C" int atlas_gdn_chunked_within(long long limit, const void* y, long long ldy, const void* a, long long lda, const void* b, long long ldb,
+                                        const float* A_log, const float* dt_bias, float* h, void* out, long long ldo,
+                                        const int* query_start_loc, const int* state_slots, const unsigned char* has_state,
+                                        const int* snap_rows, const int* snap_slots, int num_snaps_per_seq, int T, int B, int Hk, int Hv,
+                                        int Dk, int Dv, int commit, int row_lo, void* work, void* stream) {
   if (B <= 0) return 0;
   if (Dk != 128 || Dv != 128 || Hv % Hk || (ldy % 8) || (ldo % 2) || (reinterpret_cast<uintptr_t>(y) & 15) || Hv / Hk > 32) return 1;
   if (B > 65535) return 1;
@@ -642,7 +646,7 @@ extern "C" int atlas_gdn_chunked(const void* y, long long ldy, const void* a, lo
   p.B = B; p.Hk = Hk; p.Hv = Hv; p.Dv = Dv; p.commit = commit; p.scale = 1.f / sqrtf((float)Dk);
   p.row_lo = max(1, row_lo);
   int heads = 1;
-  atlas_gdn_chunked_bytes(T, B, num_snaps_per_seq, Hk, Hv, &heads);
+  atlas_gdn_chunked_bytes_within(limit, T, B, num_snaps_per_seq, Hk, Hv, &heads);
   const long long items = gdn_items(T, B, num_snaps_per_seq);
   p.mats = reinterpret_cast<float*>(work);
   p.factors = p.mats + items * heads * kGMats;
@@ -656,4 +660,12 @@ extern "C" int atlas_gdn_chunked(const void* y, long long ldy, const void* a, lo
     gdn_walk_kernel<<<dim3(p.hvn, B, Dv / kGDv), 256, sizeof(GdnSmem), st>>>(p);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
+}
+extern "C" int atlas_gdn_chunked(const void* y, long long ldy, const void* a, long long lda, const void* b, long long ldb,
+                                 const float* A_log, const float* dt_bias, float* h, void* out, long long ldo,
+                                 const int* query_start_loc, const int* state_slots, const unsigned char* has_state,
+                                 const int* snap_rows, const int* snap_slots, int num_snaps_per_seq, int T, int B, int Hk, int Hv,
+                                 int Dk, int Dv, int commit, int row_lo, void* work, void* stream) {
+  return atlas_gdn_chunked_within(kGLimit, y, ldy, a, lda, b, ldb, A_log, dt_bias, h, out, ldo, query_start_loc, state_slots, has_state, snap_rows,
+                                  snap_slots, num_snaps_per_seq, T, B, Hk, Hv, Dk, Dv, commit, row_lo, work, stream);
 }

@@ -107,6 +107,11 @@ int atlas_gdn_recurrent(const void* y, long long ldy, const void* a, long long l
                         const int* limit, const int* snap_rows, const int* snap_slots, int num_snaps_per_seq, int B,
                         int Hk, int Hv, int Dk, int Dv, int commit, int row_hi, void* stream);
 long long atlas_gdn_chunked_bytes(int T, int B, int snaps, int Hk, int Hv, int* heads);
+long long atlas_gdn_chunked_bytes_within(long long limit, int T, int B, int snaps, int Hk, int Hv, int* heads);
+int atlas_gdn_chunked_within(long long limit, const void* y, long long ldy, const void* a, long long lda, const void* b, long long ldb, const float* A_log,
+                             const float* dt_bias, float* h, void* out, long long ldo, const int* query_start_loc, const int* state_slots,
+                             const unsigned char* has_state, const int* snap_rows, const int* snap_slots, int num_snaps_per_seq, int T, int B,
+                             int Hk, int Hv, int Dk, int Dv, int commit, int row_lo, void* work, void* stream);
 int atlas_gdn_chunked(const void* y, long long ldy, const void* a, long long lda, const void* b, long long ldb, const float* A_log,
                       const float* dt_bias, float* h, void* out, long long ldo, const int* query_start_loc, const int* state_slots,
                       const unsigned char* has_state, const int* snap_rows, const int* snap_slots, int num_snaps_per_seq, int T, int B,

@@ -12,6 +12,7 @@ _vp, _ll, _i = C.c_void_p, C.c_longlong, C.c_int
 _bound = False
 USE_CHUNKED = True          # tests switch this off to compare the two kernels
 CHUNK_MIN_ROWS = 32         # rows of the longest sequence from which a step takes the chunked kernels
+WORK_LIMIT = 256 << 20      # bytes of workspace that the chunked kernels stay within, where one key head's share does
 CHUNK_ROWS_OF_SEQ = 16      # they leave sequences with fewer rows (decode rows beside a prompt) to the recurrence
 
 
@@ -25,6 +26,9 @@ def _lib():
                                           _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp]
         lib.atlas_gdn_chunked_bytes.argtypes = [_i, _i, _i, _i, _i, C.POINTER(_i)]
         lib.atlas_gdn_chunked_bytes.restype = _ll
+        lib.atlas_gdn_chunked_within.argtypes = [_ll] + lib.atlas_gdn_chunked.argtypes
+        lib.atlas_gdn_chunked_bytes_within.argtypes = [_ll] + lib.atlas_gdn_chunked_bytes.argtypes
+        lib.atlas_gdn_chunked_bytes_within.restype = _ll
         _bound = True
     return lib
 
@@ -89,12 +93,12 @@ def _run(layer, mixed, a, b, meta: _Meta, state, commit: bool):
     cuda_recurrent.conv_silu(mixed, cw, None, conv, meta, y, commit, silu=2)
     rc = 1
     if USE_CHUNKED and meta.chunk_ok and commit and layer.dk == 128 and layer.dv == 128:
-        work = torch.empty(lib.atlas_gdn_chunked_bytes(T, meta.B, meta.snaps, layer.hk, layer.hv, C.byref(_i())), dtype=torch.uint8, device=mixed.device)
-        rc = lib.atlas_gdn_chunked(y.data_ptr(), Cc, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0),
-                                   layer.A_log.data_ptr(), layer.dt_bias.data_ptr(), h.data_ptr(), out.data_ptr(),
-                                   layer.hv * layer.dv, meta.qsl.data_ptr(), meta.slots.data_ptr(), meta.has.data_ptr(),
-                                   meta.snap_rows.data_ptr(), meta.snap_slots.data_ptr(), meta.snaps, T, meta.B, layer.hk,
-                                   layer.hv, layer.dk, layer.dv, 1, CHUNK_ROWS_OF_SEQ, work.data_ptr(), st)
+        work = torch.empty(lib.atlas_gdn_chunked_bytes_within(WORK_LIMIT, T, meta.B, meta.snaps, layer.hk, layer.hv, C.byref(_i())), dtype=torch.uint8, device=mixed.device)
+        rc = lib.atlas_gdn_chunked_within(WORK_LIMIT, y.data_ptr(), Cc, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0),
+                                          layer.A_log.data_ptr(), layer.dt_bias.data_ptr(), h.data_ptr(), out.data_ptr(),
+                                          layer.hv * layer.dv, meta.qsl.data_ptr(), meta.slots.data_ptr(), meta.has.data_ptr(),
+                                          meta.snap_rows.data_ptr(), meta.snap_slots.data_ptr(), meta.snaps, T, meta.B, layer.hk,
+                                          layer.hv, layer.dk, layer.dv, 1, CHUNK_ROWS_OF_SEQ, work.data_ptr(), st)
         if rc != 1:
             K._check(rc, "gdn_chunked")
     if rc == 1 or meta.shortest < CHUNK_ROWS_OF_SEQ:           # the latter: sequences that the chunked kernels have left out

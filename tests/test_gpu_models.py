@@ -1,4 +1,6 @@
 """MoE / Gated-DeltaNet kernels and whole-model steps on the GPU against the PyTorch restatement of the same ops."""
+import ctypes
+
 import pytest
 import torch
 
@@ -139,15 +141,14 @@ def test_gdn_layer_kernels_match_reference(K):
 
 
 @pytest.mark.parametrize("split", ["1", "2", "4"])
-def test_gdn_chunked_matches_recurrence(K, split, monkeypatch):
+def test_gdn_chunked_matches_recurrence(K, split, monkeypatch):       # split: groups that the four key heads are gone through in
     """The 64-token chunked kernel (TF32 tensor cores) against the sequential recurrence kernel and the fp32 PyTorch
     recurrence: outputs, final state and mid-chunk snapshots, for sequences that start from a stored state or from
     zero, end inside a chunk, or are a single token."""
     from atlas_b200.ops import cuda_gdn
-    monkeypatch.setenv("ATLAS_GDN_SPLIT", split)       # value-column slices per head (read at every launch)
     cfg = _hybrid_cfg()
     cfg.linear_key_head_dim = cfg.linear_value_head_dim = 128
-    cfg.linear_num_key_heads, cfg.linear_num_value_heads = 2, 4
+    cfg.linear_num_key_heads, cfg.linear_num_value_heads = 4, 8
     torch.manual_seed(4)
     model = build_model(cfg, device=DEV).init_random(0)
     layer = next(l.mixer for l in model.layers if l.kind == "gdn")
@@ -161,6 +162,9 @@ def test_gdn_chunked_matches_recurrence(K, split, monkeypatch):
     b = torch.randn(T, layer.hv, device=DEV).bfloat16()
     tables = [list(range(16))] * 4
     plan = {0: [(64, 4), (144, 5)], 3: [(130, 6)]}          # 144: a snapshot row inside a chunk
+    heads = ctypes.c_int()
+    whole = cuda_gdn._lib().atlas_gdn_chunked_bytes(T, len(qlens), 2, layer.hk, layer.hv, ctypes.byref(heads))
+    monkeypatch.setattr(cuda_gdn, "WORK_LIMIT", whole // int(split))
 
     def run(chunked):
         cuda_gdn.USE_CHUNKED = chunked

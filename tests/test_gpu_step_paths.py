@@ -430,6 +430,41 @@ def test_chunked_delta_rule_workspace_is_bounded(K):
     assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
 
 
+@pytest.mark.parametrize("groups", [(2, 1), (1, 1, 1)])
+def test_chunked_delta_rule_goes_through_groups_of_heads(K, groups, monkeypatch):
+    """Three key heads of two value heads each, two and one or one at a time (a small limit in place of 256 MB): outputs, states and
+    snapshots are those of all heads at once, bit for bit, and the recurrence's."""
+    import ctypes
+    import types
+    from atlas_b200.ops import cuda_gdn
+    torch.manual_seed(3)
+    hk, hv, d, lens, plan = 3, 6, 128, [100, 7, 65], {0: [(30, 4), (64, 5)], 2: [(65, 6)]}
+    T, B, lib = sum(lens), len(lens), cuda_gdn._lib()
+    C = (2 * hk + hv) * d
+    layer = types.SimpleNamespace(hk=hk, hv=hv, dk=d, dv=d, W=4, conv_w=(torch.randn(C, 4, device=DEV) * 0.3).bfloat16(),
+                                  A_log=torch.linspace(-2, 2, hv, device=DEV), dt_bias=torch.linspace(-4, 0, hv, device=DEV))
+    mixed, a, b = (torch.randn(T, n, device=DEV).bfloat16() for n in (C, hv, hv))
+    state = dict(conv=torch.randn(8, C, 3, device=DEV).bfloat16(), h=torch.randn(8, hv, d, d, device=DEV) * 0.1)
+    meta = cuda_gdn._Meta(lens, [2, 0, 1], [True, True, False], DEV, plan)
+    heads = ctypes.c_int()
+    most = cuda_gdn.WORK_LIMIT
+    whole = lib.atlas_gdn_chunked_bytes(T, B, meta.snaps, hk, hv, ctypes.byref(heads))
+    assert heads.value == hv and whole == lib.atlas_gdn_chunked_bytes_within(most, T, B, meta.snaps, hk, hv, ctypes.byref(heads))
+    limit = whole * groups[0] // hk
+    assert lib.atlas_gdn_chunked_bytes_within(limit, T, B, meta.snaps, hk, hv, ctypes.byref(heads)) == limit and heads.value == 2 * groups[0]
+    assert lib.atlas_gdn_chunked_bytes_within(1, T, B, meta.snaps, hk, hv, ctypes.byref(heads)) == whole // hk and heads.value == 2      # never less
+    got = []
+    for lim, chunked in ((most, True), (limit, True), (most, False)):
+        monkeypatch.setattr(cuda_gdn, "WORK_LIMIT", lim)
+        monkeypatch.setattr(cuda_gdn, "USE_CHUNKED", chunked)
+        st = {k: v.clone() for k, v in state.items()}
+        got.append((cuda_gdn._run(layer, mixed, a, b, meta, st, True), st["h"], st["conv"]))
+    assert all(torch.equal(x, y) for x, y in zip(got[0], got[1]))
+    assert _rel(got[1][0], got[2][0]) < 1e-2
+    for slot in range(8):
+        assert _rel(got[1][1][slot], got[2][1][slot]) < 3e-3, slot
+
+
 # ----------------------------------------------------------------------------- chunk attention of 256-wide heads
 @pytest.mark.parametrize("kv", [torch.float8_e4m3fn, torch.bfloat16])
 @pytest.mark.parametrize("Hq,Hkv,qlens,ctxs", [(16, 2, [300, 1, 37, 63], [0, 90, 1000, 77]), (8, 2, [64, 65, 129], [64, 63, 0]), (4, 4, [130, 16], [1, 500]),
