@@ -137,17 +137,21 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bf
 // gate_up [T, 2I] -> act(gate) * up, bf16 or fp8+scale.  ACT 0: SiLU, 1: tanh-approximated GELU (Gemma).
 // `rows` (expert-sorted buffers): block i works on row rows[i], or on nothing where that is negative, so that the padding of
 // the experts' tiles costs nothing (48 tokens on 512 experts: 70 us over all padded rows, 3.3 us over the 480 live ones).
-template <int ACT>
+// LISTED: for `rows` and for blocks of several rows; a block per row in order has none of that to work out (8192 x 14336: 107.9 and 106 us).
+template <int ACT, bool LISTED>
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const __nv_bfloat16* __restrict__ gu, long long ld, int I, __nv_bfloat16* y, long long ldy, uint8_t* q,
                 long long ldq, float* scale, long long scale_ld, const int* rows, int n) {
   chain_trigger();
   chain_wait();
   // rows on grid.x: row counts can exceed the 65535 limit of grid.y; narrow rows share a block (blockDim.y whole warps of threads each)
-  const int item = (int)blockIdx.x * blockDim.y + threadIdx.y;
-  if (item >= n) return;
-  const int t = rows ? rows[item] : item;
-  if (t < 0) return;
+  int t = blockIdx.x;
+  if (LISTED) {
+    const int item = t * blockDim.y + threadIdx.y;
+    if (item >= n) return;
+    t = rows ? rows[item] : item;
+    if (t < 0) return;
+  }
   const int e = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
   const bool live = e < I;
   float o[8];
@@ -745,7 +749,7 @@ extern "C" int atlas_silu_mul(const void* gu, long long ld, int T, int I, void* 
   // large steps of narrow rows (experts): several to a block (81920 rows of 512: 86 us with a row each, 46 us so)
   const int per = T > 256 ? 256 / threads : 1;
   dim3 grid((T + per - 1) / per, (I / 8 + threads - 1) / threads);
-  launch_chain_if(T <= 256, silu_mul_kernel<0>, grid, dim3(threads, per), 0, reinterpret_cast<cudaStream_t>(stream),
+  launch_chain_if(T <= 256, rows || per > 1 ? silu_mul_kernel<0, true> : silu_mul_kernel<0, false>, grid, dim3(threads, per), 0, reinterpret_cast<cudaStream_t>(stream),
       reinterpret_cast<const __nv_bfloat16*>(gu), ld, I, reinterpret_cast<__nv_bfloat16*>(y), ldy,
       reinterpret_cast<uint8_t*>(q), ldq, scale, scale_ld, rows, T);
   return cudaGetLastError() == cudaSuccess ? 0 : -20;
@@ -756,7 +760,7 @@ extern "C" int atlas_gelu_tanh_mul(const void* gu, long long ld, int T, int I, v
   if (T <= 0) return 0;
   if (I % 8 || (q && I % 128)) return -1;
   dim3 grid(T, (I / 8 + 255) / 256);
-  launch_chain_if(T <= 256, silu_mul_kernel<1>, grid, dim3(256), 0, reinterpret_cast<cudaStream_t>(stream),
+  launch_chain_if(T <= 256, silu_mul_kernel<1, false>, grid, dim3(256), 0, reinterpret_cast<cudaStream_t>(stream),
       reinterpret_cast<const __nv_bfloat16*>(gu), ld, I, reinterpret_cast<__nv_bfloat16*>(y), ldy,
       reinterpret_cast<uint8_t*>(q), ldq, scale, scale_ld, static_cast<const int*>(nullptr), T);
   return cudaGetLastError() == cudaSuccess ? 0 : -20;
