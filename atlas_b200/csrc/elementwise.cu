@@ -529,7 +529,7 @@ v_write_pages_kernel(const RopeKvParams p) {
 
 // y = rmsnorm(x) * w * silu(z), one warp per kUnits (token, head) pairs; x, z [T, H, D] with token strides.  kPer: pairs of channels per
 // lane known at compile time (D = 64 kPer), all loads of a warp in flight together; 0: any even D.
-// Bound by memory: 8192 x 32 heads of 128 channels 106 us with a pair per warp, 72 us (2.8 TB/s).
+// Bound by memory: 8192 x 32 heads of 128 channels 103 us with a pair per warp that loads twice, 70 us (2.9 TB/s).
 template <int kPer, int kUnits>
 __global__ void __launch_bounds__(128)
 gated_rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ z,
@@ -837,9 +837,10 @@ extern "C" int atlas_gated_rmsnorm(const void* x, long long ldx, const void* z, 
                     reinterpret_cast<const __nv_bfloat16*>(x), ldx, reinterpret_cast<const __nv_bfloat16*>(z), ldz,
                     reinterpret_cast<const __nv_bfloat16*>(w), reinterpret_cast<__nv_bfloat16*>(y), ldy, T, H, D, eps);
   };
-  // four pairs a warp where that leaves every SM several blocks
+  // four pairs a warp only where memory is all that counts (16384 pairs 6.8 us with one, 7.2 with four; 65536 19.5, 19.9; 131072 36.9, 37.1;
+  // 262144 70.7, 70.2; 524288 138.7, 136.8)
   if (D != 128) run(gated_rmsnorm_kernel<0, 1>, 1);
-  else if (units >= 16384) run(gated_rmsnorm_kernel<2, 4>, 4);
+  else if (units >= 262144) run(gated_rmsnorm_kernel<2, 4>, 4);
   else run(gated_rmsnorm_kernel<2, 1>, 1);
   return cudaGetLastError() == cudaSuccess ? 0 : -20;
 }

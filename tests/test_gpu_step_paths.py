@@ -136,7 +136,7 @@ def test_route_picks_the_largest(K, E, k, dtype):
     assert float((w.double() - want).abs().max()) < 1e-5
 
 
-@pytest.mark.parametrize("T,H,D", [(1, 3, 128), (7, 5, 128), (600, 31, 128), (513, 32, 128), (5, 3, 96)])
+@pytest.mark.parametrize("T,H,D", [(1, 3, 128), (7, 5, 128), (600, 31, 128), (513, 32, 128), (5, 3, 96), (8193, 32, 128)])
 def test_gated_norm_of_heads(K, T, H, D):
     torch.manual_seed(T)
     x, z, w = (torch.randn(*s, device=DEV).bfloat16() for s in ((T, H, D), (T, H, D), (D,)))
