@@ -280,6 +280,32 @@ class ModelRunner:
         return g.run(batch)
 
 
+def _capture(stream: "torch.cuda.Stream", fn):
+    """``(graph, result)`` of ``fn`` captured on ``stream``.  The request whose step meets a batch size first waits for this, so the cached
+    blocks are given back and garbage is collected only where memory is short (a step of one Gated DeltaNet row, four layers: 160 to
+    460 ms with both, 19 without).  Nothing is collected during the capture: that could destroy events, pinned buffers or graphs of
+    other engines, which a capturing stream forbids."""
+    free, total = torch.cuda.mem_get_info()
+    if free < total // 16:
+        gc.collect()
+        torch.cuda.empty_cache()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    collecting = gc.isenabled()
+    gc.disable()
+    try:
+        with torch.cuda.stream(stream):
+            graph.capture_begin()
+            try:
+                out = fn()
+            finally:
+                graph.capture_end()
+    finally:
+        if collecting:
+            gc.enable()
+    return graph, out
+
+
 class _DecodeGraph:
     """One captured decode step for a padded batch size; inputs are copied into fixed buffers."""
 
@@ -341,21 +367,10 @@ class _DecodeGraph:
                 for _ in range(2):
                     r.model.forward(fb, r.cache)
             torch.cuda.current_stream().wait_stream(s)
-            self.graph = torch.cuda.CUDAGraph()
             from .ops import cuda as K
             K.freeze_scratch()
             n0 = K.launch_count
-            # a collection during the capture could destroy events, pinned buffers or graphs of other engines, which the
-            # capturing stream forbids
-            gc.collect()
-            collecting = gc.isenabled()
-            gc.disable()
-            try:
-                with torch.cuda.graph(self.graph):
-                    self.out = r.model.forward(fb, r.cache)
-            finally:
-                if collecting:
-                    gc.enable()
+            self.graph, self.out = _capture(s, lambda: r.model.forward(fb, r.cache))
             self.num_kernels = K.launch_count - n0
             self._load(b)
         self.graph.replay()

@@ -344,6 +344,27 @@ def test_delta_net_decode_graph_equals_eager_steps(K, n):
     assert all(torch.equal(a, b) for a, b in zip(*outs))
 
 
+@pytest.mark.parametrize("short", [False, True])
+def test_capture_gives_memory_back_only_where_it_is_short(K, short, monkeypatch):
+    """The first step of a batch size pays for two eager passes and a capture, not for a collection and the allocator's cache."""
+    import gc
+    from atlas_b200 import runner
+    calls = []
+    total = torch.cuda.mem_get_info()[1]
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (total // 32 if short else total // 2, total))
+    monkeypatch.setattr(gc, "collect", lambda *a: calls.append("collect"))
+    monkeypatch.setattr(torch.cuda, "empty_cache", lambda: calls.append("empty"))
+    x = torch.arange(8.0, device=DEV)
+    graph, y = runner._capture(torch.cuda.Stream(), lambda: x * 2)
+    assert gc.isenabled() and calls == (["collect", "empty"] if short else [])
+    x.add_(1)
+    graph.replay()
+    assert torch.equal(y, (torch.arange(8.0, device=DEV) + 1) * 2)
+    with pytest.raises(ZeroDivisionError):
+        runner._capture(torch.cuda.Stream(), lambda: x * (1 // 0))
+    assert gc.isenabled() and float((x + 1).sum()) == 44.0          # the stream is usable again
+
+
 # ----------------------------------------------------------------------------- chunked delta rule
 def _delta_rule(y, a, b, a_log, dt_bias, h, hk, hv, stops):
     """The recurrence in 64 bits: outputs, and the state after every row count in ``stops``."""
