@@ -503,3 +503,33 @@ def test_chunk_attention_of_wide_heads(K, kv, Hq, Hkv, qlens, ctxs, monkeypatch)
     old, _ = _attention_case(K, 256, Hq, Hkv, **args)
     assert _rel(out, want) <= 1.05 * _rel(old, want)
     assert _rel(out, old) < 2e-2
+
+
+@pytest.mark.parametrize("opts", [dict(window=40), dict(window=64, sinks=True), dict(chunk=96), dict(chunk=64, sinks=True), dict(softcap=5.0, sinks=True),
+                                  dict(distance=17), dict(distance=700), dict(distance=9, sinks=True, window=50), dict(distance=30, softcap=8.0)])
+@pytest.mark.parametrize("Hq,Hkv", [(4, 4), (6, 2), (16, 2), (20, 1)])
+def test_chunk_attention_of_wide_heads_with_every_option(K, Hq, Hkv, opts, monkeypatch):
+    """Head dim 256, bf16 cache: windows, chunked visibility, sinks, bounded scores and distance biases (in shared memory and too many for
+    it) on the tcgen05 tiles and on the general kernel.  Both round P and the result to bf16, at other places: 2^-8 each at most."""
+    g = torch.Generator(device=DEV).manual_seed(Hq)
+    qlens, ctxs, D = [130, 5, 64, 33], [0, 300, 63, 127], 256
+    nblk = [(c + n + 15) // 16 for c, n in zip(ctxs, qlens)]
+    perm, tables, off = torch.randperm(sum(nblk) + 2, generator=g, device=DEV).tolist(), [], 0
+    for n in nblk:
+        tables.append(perm[off:off + n])
+        off += n
+    kc, vc = K.alloc_kv_cache(sum(nblk) + 2, 16, Hkv, D, torch.bfloat16, DEV)
+    kc.copy_(torch.randn(kc.shape, generator=g, device=DEV).bfloat16())
+    vc.copy_(torch.randn(vc.shape, generator=g, device=DEV).bfloat16())
+    q = torch.randn(sum(qlens), Hq, D, generator=g, device=DEV).bfloat16()
+    sinks = torch.randn(Hq, generator=g, device=DEV) if opts.get("sinks") else None
+    reach = opts.get("distance")
+    distance = torch.randn(Hq, reach + 1, generator=g, device=DEV) if reach else None
+    outs = []
+    for tc in (True, False):
+        monkeypatch.setattr(K, "_TC_PREFILL", tc)
+        fb = ForwardBatch.build([[0] * n for n in qlens], ctxs, tables, 16, device=DEV)
+        outs.append(K.paged_attention(q, kc, vc, fb, D ** -0.5, 1.0, 1.0, opts.get("window"), opts.get("chunk", 0), sinks, opts.get("softcap", 0.0), distance))
+    assert K.check_status() == 0
+    assert _rel(outs[0], outs[1]) < 2 ** -7
+    torch.testing.assert_close(outs[0].float(), outs[1].float(), atol=3e-2, rtol=3e-2)
