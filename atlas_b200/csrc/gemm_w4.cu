@@ -31,8 +31,8 @@ constexpr int kW4Threads = 32 * (2 + kW4ConvWarps + kW4EpiWarps + 1);
 constexpr int kW4AWarp = 2 + kW4ConvWarps + kW4EpiWarps;      // index of the A-tile producer warp
 
 // ROWS 256: two row tiles share every converted slice.  What bounds a slice of one tile is its conversion (ALU work of eight warps, three to
-// four times the MMAs): 8192 x 4096 x 4096 445 us with one tile, 292 us with two; 36016 routed rows on 128 experts of 1536 x 2048 and
-// 2048 x 768 741 and 652 us for the pair of products.
+// four times the MMAs): 8192 x 4096 x 4096 445 us with one tile, 313 us with two; 36016 routed rows on 128 experts of 1536 x 2048 and
+// 2048 x 768 827 and 670 us for the pair of products (cold).
 template <int BLOCK_N, int ROWS>
 struct W4Cfg {
   static constexpr int kTiles = ROWS / kW4BlockM;
@@ -92,7 +92,7 @@ struct W4Work { int t0, count, n_tile; };
 template <int TILES, typename F>
 ATLAS_DEVICE bool w4_unit(const W4Params& p, int item, int m_tiles, F work) {
   // Experts: the column tiles of a unit one after the other, so that its rows come from HBM once and from L2 after that (row tiles
-  // first read 190 MB of rows again for every column tile: the pair of products 652, so 567 us).
+  // first read 190 MB of rows again for every column tile: an expert layer of 6000 tokens x 8 of those 128, 971 us, so 840).
   if (p.tile_expert) {
     const int u = item / p.n_tiles, t0 = TILES == 1 ? u : p.unit_tile[u];
     const bool two = TILES == 2 && t0 + 1 < m_tiles && p.tile_expert[t0] == p.tile_expert[t0 + 1];

@@ -533,3 +533,69 @@ def test_chunk_attention_of_wide_heads_with_every_option(K, Hq, Hkv, opts, monke
     assert K.check_status() == 0
     assert _rel(outs[0], outs[1]) < 2 ** -7
     torch.testing.assert_close(outs[0].float(), outs[1].float(), atol=3e-2, rtol=3e-2)
+
+
+# ----------------------------------------------------------------------------- wide tiles whose last one is cut off
+@pytest.mark.parametrize("N", [1990, 2040, 1947])
+@pytest.mark.parametrize("form", ["plain", "bias", "unit", "unit_tail", "relu2", "tail", "tail_bias"])
+def test_bf16_products_on_cut_off_wide_tiles(K, N, form):
+    """38 row tiles of 128 on 256-wide column tiles of which the last one is not whole, through every epilogue, against fp32 products of the
+    same bf16 values (fp32 sums; results rounded to bf16: 2^-9, a gated unit's two factors before that)."""
+    g = torch.Generator(device=DEV).manual_seed(N)
+    M, Kd = 4737, 136
+    if form.startswith("unit"):
+        N = N // 16 * 16
+    assert K.gemm_plan(M, N, Kd, 0, 148)[0] == 256 and N % 256
+    x = torch.randn(M, Kd, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(N, Kd, generator=g, device=DEV) * 0.1).bfloat16()
+    bias = torch.randn(N, generator=g, device=DEV)
+    want = x.double() @ w.double().t()
+    unit, n_main = (7.0, 1.702, 1.0), N - 80
+
+    def gated(v):
+        gate, up = v[:, 0::2].clamp(max=unit[0]), v[:, 1::2].clamp(-unit[0], unit[0])
+        return gate * torch.sigmoid(unit[1] * gate) * (up + unit[2])
+
+    if form == "plain":
+        pairs = [(K.gemm_bf16(x, w), want)]
+    elif form == "bias":
+        pairs = [(K.gemm_bf16(x, w, bias=bias), want + bias.double())]
+    elif form == "unit":
+        pairs = [(K.gemm_bf16(x, w, unit=unit), gated(want))]
+    elif form == "unit_tail":
+        main, tail = K.gemm_bf16(x, w, unit=unit, n_main=n_main)
+        pairs = [(main, gated(want[:, :n_main])), (tail, want[:, n_main:])]
+    elif form == "relu2":
+        pairs = [(K.gemm_bf16(x, w, relu2_cols=N - 70), torch.cat([want[:, :N - 70].relu().square(), want[:, N - 70:]], 1))]
+    else:
+        b = bias if form == "tail_bias" else None
+        main, tail = K.linear_tail(x, w, N - 77, b)
+        full = want + (bias.double() if b is not None else 0.0)
+        pairs = [(main, full[:, :N - 77]), (tail, full[:, N - 77:])]
+    assert K.check_status() == 0
+    for got, ref64 in pairs:
+        assert got.shape == ref64.shape and _rel(got, ref64) < (2 ** -9 if got.dtype == torch.bfloat16 else 1e-5)
+        assert float((got.double() - ref64)[:, -16:].abs().max()) < 2 ** -6 * float(ref64.abs().max())
+
+
+@pytest.mark.parametrize("M,N,Kd", [(4737, 1984, 2048), (4737, 2000, 4096), (300, 18432 + 136, 6144)])
+def test_fp8_products_on_cut_off_wide_tiles(K, M, N, Kd):
+    """Block scales of the last, half or fully missing 128 columns of a wide tile: against 64 bits with the same scales."""
+    g = torch.Generator(device=DEV).manual_seed(N)
+    xq, xs = K.quant_fp8(torch.randn(M, Kd, generator=g, device=DEV).bfloat16())
+    w = torch.randn(N, Kd, generator=g, device=DEV).to(torch.float8_e4m3fn)
+    ws = torch.rand((N + 127) // 128, Kd // 128, generator=g, device=DEV) + 0.5
+    got = {}
+    for bn in (256, 128):
+        plan = K.gemm_plan
+        try:
+            K.gemm_plan = lambda *a: (bn, 1)
+            got[bn] = K.gemm_fp8_block(xq, xs, w, ws)
+        finally:
+            K.gemm_plan = plan
+    assert K.check_status() == 0
+    assert torch.equal(got[256], got[128])
+    rows = torch.tensor([0, 1, M // 2, M - 1], device=DEV)
+    a = xq[rows].double().view(4, -1, 128) * xs[rows].double()[..., None]
+    b = w.double().view(N, -1, 128) * ws.double().repeat_interleave(128, 0)[:N, :, None]
+    assert _rel(got[256][rows], a.flatten(1) @ b.flatten(1).t()) < 2 ** -9
