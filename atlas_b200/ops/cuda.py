@@ -311,8 +311,10 @@ def gemm_plan(M: int, N: int, K: int, kind: int, sms: int) -> Tuple[int, int]:
     m_tiles = (M + 127) // 128
     if _FORCE_BLOCK_N:
         bn = _FORCE_BLOCK_N
-    elif kind == 0 and m_tiles * ((N + 255) // 256) >= 2 * sms and -N % 256 * 16 <= N:
-        bn = 256          # bf16 accumulates in TMEM across K; a last tile that is cut off costs at most 1/16
+    elif kind == 0 and m_tiles * ((N + 255) // 256) >= 2 * sms and (N % 256 == 0 or (K > 128 and -N % 256 * 16 <= N)):
+        # bf16 accumulates in TMEM across K; a last tile that is cut off costs at most 1/16 (8192 x 12352: K 128 132 us narrow, 138 wide; 1024
+        # 260 and 207; 4096 925 and 663)
+        bn = 256
     elif kind == 1 and m_tiles * ((N + 255) // 256) >= sms and (N % 256 == 0 or _wide_cut_pays(m_tiles, N, K, sms)):
         bn = 256          # fp8: half the per-k-group buffer handshakes per FLOP and 0.75x the shared-memory fill of 128
     elif m_tiles * ((N + 127) // 128) >= sms:

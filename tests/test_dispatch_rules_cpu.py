@@ -17,6 +17,11 @@ def test_bf16_decode_products_of_long_k(M, N, Kd, want):
     assert K.gemm_plan(M, N, Kd, 0, SMS) == want
 
 
+@pytest.mark.parametrize("M,N,Kd,want", [(8192, 12352, 128, 128), (8192, 12352, 136, 256), (8192, 12288, 64, 256), (8192, 1921, 4096, 128)])
+def test_bf16_products_whose_last_wide_tile_is_cut_off(M, N, Kd, want):
+    assert K.gemm_plan(M, N, Kd, 0, SMS)[0] == want
+
+
 @pytest.mark.parametrize("M,N,Kd,want", [
     (4500, 12352, 1024, 128), (8192, 18560, 1536, 128),                     # a wide tile of short K costs more than two narrow ones
     (4500, 12352, 2048, 256), (8192, 12352, 2048, 128), (8192, 12352, 4096, 256), (2500, 4992, 2048, 256),
